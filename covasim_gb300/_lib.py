@@ -175,6 +175,11 @@ def lib():
         L.covgpu_infections_scratch_bytes.restype = i64
         L.covgpu_infections.argtypes = [f32, vp, vp, vp, i64, vp, vp, i64, vp, u64, i32, i32, i32, vp, vp, i64, vp,
                                         vp, vp, i64, vp]
+        L.covgpu_infections_find.argtypes = [f32, vp, vp, vp, i64, vp, vp, i64, vp, u64, i32, i32, i32, vp, vp, vp,
+                                             i64, vp]
+        L.covgpu_infections_find.restype = C.c_int
+        L.covgpu_infections_emit.argtypes = [vp, vp, i64, vp, i64, vp, vp, vp]
+        L.covgpu_infections_emit.restype = C.c_int
         L.covgpu_infections_noalloc.argtypes = [f32, vp, vp, vp, i64, vp, vp, i64, vp, u64, i32, i32, i32, vp, vp,
                                                 i64, vp, vp, vp]
         L.covgpu_infections_noalloc.restype = C.c_int
@@ -248,7 +253,8 @@ POP_FUNCS = ['covgpu_pop_ages', 'covgpu_pop_members', 'covgpu_pop_random_counts'
              'covgpu_pop_cluster_sizes', 'covgpu_pop_cluster_counts', 'covgpu_pop_cluster_fill', 'covgpu_pop_prognoses']
 
 EXPORTED = ['covgpu_version', 'covgpu_abi_layout', 'covgpu_viral_load', 'covgpu_trans_sus', 'covgpu_infections_scratch_bytes',
-            'covgpu_infections', 'covgpu_infections_noalloc', 'covgpu_agent_step', 'covgpu_edge_pass', 'covgpu_infect_claims',
+            'covgpu_infections', 'covgpu_infections_find', 'covgpu_infections_emit',
+            'covgpu_infections_noalloc', 'covgpu_agent_step', 'covgpu_edge_pass', 'covgpu_infect_claims',
             'covgpu_infect_list', 'covgpu_import_day', 'covgpu_rescale_check', 'covgpu_layer_lists', 'covgpu_run_days', 'covgpu_test_trace',
             'covgpu_lik_targets', 'covgpu_trace_index_scratch', 'covgpu_trace_index', 'covgpu_edge_resident_bytes',
             'covgpu_check', 'covgpu_check_immunity', 'covgpu_update_nab', 'covgpu_update_peak_nab',

@@ -36,32 +36,6 @@ using namespace covgpu;
 
 namespace {
 
-// Programmatic dependent launch for the day's kernels: a kernel launched with
-// launch_pdl may be scheduled while its stream predecessor's last blocks finish
-// (inside a captured graph the edge becomes a programmatic one); pdl_wait, the
-// first statement of each such kernel, holds it until the predecessor has
-// completed and its writes are visible. Launched the ordinary way, pdl_wait
-// returns at once.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// A block's signal that the next kernel's blocks may be scheduled once every block
-// of this grid has given it or exited: their set-up before pdl_wait (tables,
-// read-only descriptors) then overlaps this grid's last blocks.
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-template <typename... K, typename... A>
-void launch_pdl(void (*kernel)(K...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 // resident blocks per SM that the register budget of the agent pass must allow
 // (0: the compiler's choice); the pass's grid is one wave of them. Three blocks
 // ran a whole 1M-agent run (one CUDA graph) 0.8 ms faster than four and 2.3 ms

@@ -45,6 +45,32 @@ inline unsigned wave_grid(const covgpu_state* st, int64_t wave) {
   return (unsigned)(nb < wave ? (nb > 0 ? nb : 1) : wave);
 }
 
+// Programmatic dependent launch: a kernel launched with
+// launch_pdl may be scheduled while its stream predecessor's last blocks finish
+// (inside a captured graph the edge becomes a programmatic one); pdl_wait, the
+// first statement of each such kernel, holds it until the predecessor has
+// completed and its writes are visible. Launched the ordinary way, pdl_wait
+// returns at once.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A block's signal that the next kernel's blocks may be scheduled once every block
+// of this grid has given it or exited: their set-up before pdl_wait (tables,
+// read-only descriptors) then overlaps this grid's last blocks.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... K, typename... A>
+void launch_pdl(void (*kernel)(K...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // the checks every state entry point makes before launching (covgpu.cu)
 int check_state(const covgpu_state* st);
 // the testing, tracing and post passes of day t (covgpu_testing.cu)

@@ -64,20 +64,22 @@ def _infections_op(beta: float, p1: torch.Tensor, p2: torch.Tensor, layer_betas:
                    variant: int, layer: int) -> tuple[torch.Tensor, torch.Tensor]:
     E = p1.numel()
     dev = p1.device
-    cap = 2 * E
-    src = torch.empty(max(cap, 1), dtype=_I32, device=dev)
-    tgt = torch.empty(max(cap, 1), dtype=_I32, device=dev)
-    count = torch.zeros(1, dtype=torch.int64, device=dev)
-    status = torch.zeros(1, dtype=_I32, device=dev)
+    if E == 0:
+        return torch.empty(0, dtype=_I32, device=dev), torch.empty(0, dtype=_I32, device=dev)
+    n_agents = min(rel_trans.numel(), rel_sus.numel())
+    count = torch.zeros(2, dtype=torch.int64, device=dev)  # transmissions, status
     nbytes = int(L.lib().covgpu_infections_scratch_bytes(E))
     scratch = torch.empty(nbytes, dtype=_U8, device=dev)
-    L.call('covgpu_infections', float(np.float32(beta)), _ptr(p1), _ptr(p2), _ptr(layer_betas), E, _ptr(rel_trans),
-           _ptr(rel_sus), min(rel_trans.numel(), rel_sus.numel()), _ptr(uniforms), int(seed) & 0xFFFFFFFFFFFFFFFF, int(day), int(variant), int(layer),
-           _ptr(src), _ptr(tgt), cap, _ptr(count), _ptr(status), scratch.data_ptr(), nbytes, _stream())
-    n = int(count.item())
-    if int(status.item()) & L.BADARG:
+    L.call('covgpu_infections_find', float(np.float32(beta)), _ptr(p1), _ptr(p2), _ptr(layer_betas), E,
+           _ptr(rel_trans), _ptr(rel_sus), n_agents, _ptr(uniforms), int(seed) & 0xFFFFFFFFFFFFFFFF, int(day),
+           int(variant), int(layer), count.data_ptr(), count.data_ptr() + 8, scratch.data_ptr(), nbytes, _stream())
+    n, status = count.tolist()
+    if status & L.BADARG:
         raise IndexError('compute_infections: an edge index is outside the agent arrays')
-    return src[:n].clone(), tgt[:n].clone()
+    src = torch.empty(n, dtype=_I32, device=dev)
+    tgt = torch.empty(n, dtype=_I32, device=dev)
+    L.call('covgpu_infections_emit', _ptr(p1), _ptr(p2), E, scratch.data_ptr(), n, _ptr(src), _ptr(tgt), _stream())
+    return src, tgt
 
 
 # ---------------------------------------------------------------- reference-signature drop-ins

@@ -412,13 +412,29 @@ int covgpu_trans_sus(const float* rel_trans, const float* rel_sus, const uint8_t
  * the first capacity are written and COVGPU_OVERFLOW is stored in *status.
  * An edge whose p1 or p2 is outside [0, n_agents) is skipped and
  * COVGPU_BADARG is stored in *status (status may be NULL).
- * scratch: device memory of covgpu_infections_scratch_bytes(n_edges) bytes. */
+ * scratch: device memory of covgpu_infections_scratch_bytes(n_edges) bytes.
+ * (24 bytes per 2048 edges plus 256 are accepted too: then every edge is
+ * evaluated twice instead of once.) */
 int64_t covgpu_infections_scratch_bytes(int64_t n_edges);
 int covgpu_infections(float beta, const int32_t* p1, const int32_t* p2, const float* layer_betas,
                       int64_t n_edges, const float* rel_trans, const float* rel_sus, int64_t n_agents,
                       const double* uniforms, uint64_t seed, int32_t day, int32_t variant, int32_t layer,
                       int32_t* out_src, int32_t* out_tgt, int64_t capacity, int64_t* out_count,
                       int32_t* status, void* scratch, int64_t scratch_bytes, void* stream);
+
+/* compute_infections in two calls, for callers that allocate outputs of the
+ * exact size: _find evaluates every edge (1 <= n_edges <= 2^36), adds the
+ * number of transmissions to *out_count and ORs COVGPU_BADARG into *status
+ * for a bad edge (device, cleared by the caller; status may be NULL); _emit
+ * then writes the first `count` transmissions from the same scratch, which
+ * must not change in between. scratch: covgpu_infections_scratch_bytes(n_edges)
+ * bytes. */
+int covgpu_infections_find(float beta, const int32_t* p1, const int32_t* p2, const float* layer_betas,
+                           int64_t n_edges, const float* rel_trans, const float* rel_sus, int64_t n_agents,
+                           const double* uniforms, uint64_t seed, int32_t day, int32_t variant, int32_t layer,
+                           int64_t* out_count, int32_t* status, void* scratch, int64_t scratch_bytes, void* stream);
+int covgpu_infections_emit(const int32_t* p1, const int32_t* p2, int64_t n_edges, const void* scratch,
+                           int64_t count, int32_t* out_src, int32_t* out_tgt, void* stream);
 
 /* compute_infections for callers that cannot allocate device memory. (No
  * counterpart in the reference, which has no device memory at all.) Some
