@@ -19,8 +19,10 @@ namespace {
 //
 // Day t with a test_prob / contact_tracing sim, after the agent pass and any
 // importations (sim.py:596-600): k_test_pass draws who tests and marks the
-// agents to trace, k_trace_scan marks their contacts layer by layer, and
-// k_post_pass notifies the contacts and runs update_states_post.
+// contacts of the agents to trace, and k_post_pass notifies the contacts and runs
+// update_states_post. A tracing capacity, or a stored layer without an index, takes
+// the marking out of the test pass: k_trace_cap, k_trace_scan and k_trace_marks
+// then work from its bitmap of the traced.
 
 __device__ __forceinline__ bool day_active(int t, int start, int end) { return t >= start && t <= end; }
 
@@ -69,12 +71,70 @@ __device__ __forceinline__ uint64_t swab_threshold(const covgpu_state& st, const
   return prob_thr(__dmul_rn(__dmul_rn(T.swab_pdf[d], adj), cnt));
 }
 
+// contact_tracing.identify_contacts, the find_contacts half (utils.py:131-147), for
+// the traced agents of one warp's 32 (bit r of `traced`: agent i0 + r): each marks
+// the other endpoint of its edges in the layers' bitmaps. A traced agent's layers
+// are spread over four groups of eight lanes, whose lanes share its edges: as p1
+// and p2 through a stored layer's index, and the partners of its two lists (the
+// draws the edge pass makes for that agent as a source) in a redrawn layer. The
+// chain of dependent loads (row, edge, endpoint) is paid about once per traced
+// agent instead of once per edge. In a 300,000-agent sim (a median day): the test
+// pass with the marks 17.0 us, against 7.8 us without them, 21.1 us for a thread of
+// its own per traced agent and 12.4 us for the redrawn layer's lists, three
+// launches.
+constexpr int MARK_LANES = 8;
+__device__ __noinline__ void mark_contacts(const covgpu_state& st, const covgpu_sim_params& sp, int64_t i0, uint32_t traced, int t) {
+  const covgpu_testing& T = sp.testing;
+  const int lane = threadIdx.x & 31, sub = lane & (MARK_LANES - 1);
+  const int64_t words = (st.n + 31) >> 5;
+  const int32_t off = (int32_t)sp.agent_off;
+  const uint32_t n_local = (uint32_t)sp.n_agents;
+  for (; traced; traced &= traced - 1) {
+    const uint32_t a = (uint32_t)(i0 + (__ffs(traced) - 1) - off);
+    for (int l = lane / MARK_LANES; l < sp.n_layers; l += 32 / MARK_LANES) {
+      const int seg = sp.seg_of_layer[l];
+      if (seg < 0 || T.thr_trace[l] == 0) continue;
+      const covgpu_layer& L = st.segments[seg];
+      uint32_t* contact = st.contact_bits + (int64_t)l * words;
+      if (L.dynamic) {
+        int k[2];
+        dyn_counts(L.dyn_cdf, L.dyn_k, a, (uint32_t)t, (uint32_t)l, sp.key0, sp.key1, k[0], k[1]);
+        const uint32_t thr = bounded_thr(n_local);
+        const int nb0 = (k[0] + 3) >> 2, nb = nb0 + ((k[1] + 3) >> 2);  // four-entry blocks of both lists
+        for (int b = sub; b < nb; b += MARK_LANES) {
+          const int d = b >= nb0 ? 1 : 0, j0 = 4 * (d ? b - nb0 : b);
+          const uint4 pw = dyn_partner_block(a, d, j0, (uint32_t)t, (uint32_t)l, sp.key0, sp.key1);
+          for (int j = j0; j < j0 + 4 && j < k[d]; ++j) {
+            const int32_t g = off + (int32_t)dyn_partner(word_of(pw, j & 3), n_local, thr, a, d, j, (uint32_t)t,
+                                                         (uint32_t)l, sp.key0, sp.key1);
+            atomicOr(contact + (g >> 5), 1u << (g & 31));
+          }
+        }
+      } else if (L.rp1) {
+        const uint32_t b1 = L.rp1[a], e1 = L.rp1[a + 1], b2 = L.rp2[a], e2 = L.rp2[a + 1];
+        for (uint32_t k = b1 + sub; k < e1; k += MARK_LANES) {
+          const int32_t g = L.p2[k];
+          atomicOr(contact + (g >> 5), 1u << (g & 31));
+        }
+        for (uint32_t k = b2 + sub; k < e2; k += MARK_LANES) {
+          const int32_t g = L.p1[L.perm2[k]];
+          atomicOr(contact + (g >> 5), 1u << (g & 31));
+        }
+      }
+    }
+    __syncwarp();
+  }
+}
+
 // test_prob.apply (interventions.py:921-981) + People.test (people.py:589-617),
-// then the trace bits of contact_tracing.select_cases (interventions.py:1066-1072)
-// One agent block of the test pass (thread k on agent begin + k); the tested are
-// counted into the thread's accumulator
-__device__ __forceinline__ void test_block(const covgpu_state& st, int t, const covgpu_agent_block& blk,
-                                           unsigned& tested_acc) {
+// then the agents contact_tracing.select_cases picks (interventions.py:1066-1072).
+// One agent block of the test pass (thread k on agent begin + k, its flags f and
+// diagnosis date dd already loaded); the tested are counted into the thread's
+// accumulator. MARK: the traced agents' contacts are marked here, else the traced
+// go to their bitmap.
+template <bool MARK>
+__device__ __forceinline__ void test_block(const covgpu_state& st, int t, const covgpu_agent_block& blk, uint32_t f,
+                                           float dd, unsigned& tested_acc) {
   const covgpu_sim_params& sp = st.sims[blk.sim];
   const covgpu_testing& T = sp.testing;
   const bool test_on = day_active(t, T.test_start, T.test_end);
@@ -85,19 +145,18 @@ __device__ __forceinline__ void test_block(const covgpu_state& st, int t, const 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t tested = 0, trace = 0;
   if (valid) {
-    uint32_t f = st.flags[i];
-    float* d_diag = date_row(st, COVGPU_DATE_DIAGNOSED) + i;
-    float dd = *d_diag;  // loaded with the flags; kept current below
     if (test_on) {
       uint64_t thr = 0;
       if (!(f & B_DIAG)) {  // the diagnosed do not test
         const bool symp = f & B_SYMP;
         const int64_t loc = i - sp.agent_off;
+        // quarantined testers with everyone's probabilities need not be told apart
+        const bool quar_differs = T.swab_pdf || T.thr_symp_quar != T.thr_symp || T.thr_asymp_quar != T.thr_asymp;
         // an influenza-like illness without COVID symptoms: the symptomatic probability,
         // never the quarantine ones (interventions.py:966-969)
         if (!symp && T.ili_mark && T.ili_mark[loc] == t)
           thr = T.thr_symp;
-        else if (quar_tester(st, T, i, t, f))
+        else if (quar_differs && quar_tester(st, T, i, t, f))
           thr = symp ? T.thr_symp_quar : T.thr_asymp_quar;
         else
           thr = !symp ? T.thr_asymp : (T.swab_pdf ? swab_threshold(st, T, i, t) : T.thr_symp);
@@ -117,7 +176,7 @@ __device__ __forceinline__ void test_block(const covgpu_state& st, int t, const 
             const uint4 w1 = philox(make_uint4(local, 1u, (uint32_t)t, TAG_TEST), sp.key0, sp.key1);
             if (bern52_thr(w1.x, w1.y, T.thr_not_lost)) {
               dd = (float)(t + T.test_delay);
-              *d_diag = dd;
+              date_row(st, COVGPU_DATE_DIAGNOSED)[i] = dd;
               date_row(st, COVGPU_DATE_POS_TEST)[i] = (float)t;
             }
           }
@@ -131,7 +190,12 @@ __device__ __forceinline__ void test_block(const covgpu_state& st, int t, const 
         trace = (dd == (float)t) ? 1u : 0u;
     }
   }
+  tested_acc += tested;
   const uint32_t tm = __ballot_sync(0xffffffffu, trace);
+  if (MARK) {
+    if (tm) mark_contacts(st, sp, blk.begin + warp * 32, tm, t);
+    return;
+  }
   if (trace_on && lane == 0 && blk.begin + warp * 32 < blk.end) st.trace_bits[(blk.begin + warp * 32) >> 5] = tm;
   if (tm && T.cap_list) {  // the day's cases, for the capacity's selection (k_trace_cap)
     uint32_t base = 0u;
@@ -139,7 +203,6 @@ __device__ __forceinline__ void test_block(const covgpu_state& st, int t, const 
     base = __shfl_sync(0xffffffffu, base, 0);
     if (trace) T.cap_list[base + __popc(tm & ((1u << lane) - 1u))] = (int32_t)(i - sp.agent_off);
   }
-  tested_acc += tested;
   if (lane == 0 && tm) atomicAdd(st.trace_count + blk.sim, (unsigned)__popc(tm));
 }
 
@@ -260,7 +323,17 @@ __global__ void k_trace_cap(covgpu_state st, int t) {
   if (threadIdx.x == 0) st.trace_count[s] = (uint32_t)cap;
 }
 
-__global__ void __launch_bounds__(AGENT_THREADS) k_test_pass(covgpu_state st, int t) {
+// The test and post passes wait on memory (8 and 16 bytes an agent, little
+// arithmetic), so they run at full occupancy: eight blocks of 32 registers per SM.
+// On the 10M-agent testing run (the 80 days after the last variant's arrival):
+// 99.3 ms, against 103.5 ms with six blocks (two agent blocks loaded at a time),
+// 111.7 ms with four (four at a time) and 115.0 ms with three. A day of it, test
+// 111 -> 73 us (marks included), post 172 -> 95 us: the bytes take 12 and 24 us.
+constexpr int PASS_BLOCKS = 8;
+
+template <bool MARK>
+__global__ void __launch_bounds__(AGENT_THREADS, PASS_BLOCKS) k_test_pass(covgpu_state st, int t) {
+  pdl_wait();
   if (held(st, t)) return;
   int64_t b, b_end;
   if (!agent_range(st, b, b_end)) return;
@@ -268,13 +341,40 @@ __global__ void __launch_bounds__(AGENT_THREADS) k_test_pass(covgpu_state st, in
   unsigned tested_acc = 0;
   for (; b < b_end; ++b) {
     const covgpu_agent_block blk = st.agent_blocks[b];
+    const int64_t i = blk.begin + threadIdx.x;
+    uint32_t f = 0u;
+    float dd = 0.0f;
+    if (i < blk.end) {
+      f = st.flags[i];
+      dd = date_row(st, COVGPU_DATE_DIAGNOSED)[i];
+    }
     if (blk.sim != sim) {
       test_flush(st, t, sim, tested_acc);
       sim = blk.sim;
     }
-    test_block(st, t, blk, tested_acc);
+    test_block<MARK>(st, t, blk, f, dd, tested_acc);
   }
+  pdl_trigger();
   test_flush(st, t, sim, tested_acc);
+}
+
+// The marking on its own, from the test pass's bitmap of the traced (after the
+// capacity's selection): one warp per agent block's word
+__global__ void __launch_bounds__(AGENT_THREADS) k_trace_marks(covgpu_state st, int t) {
+  if (held(st, t)) return;
+  int64_t b, b_end;
+  if (!agent_range(st, b, b_end)) return;
+  const int warp = threadIdx.x >> 5;
+  for (; b < b_end; ++b) {
+    const covgpu_agent_block blk = st.agent_blocks[b];
+    const covgpu_sim_params& sp = st.sims[blk.sim];
+    const int64_t i0 = blk.begin + warp * 32;
+    if (i0 >= blk.end || !day_active(t, sp.testing.trace_start, sp.testing.trace_end) ||
+        st.trace_count[blk.sim] == 0)
+      continue;
+    const uint32_t tm = st.trace_bits[i0 >> 5];
+    if (tm) mark_contacts(st, sp, i0, tm, t);
+  }
 }
 
 __device__ __forceinline__ uint32_t bit_of(const uint32_t* __restrict__ bits, int32_t a) {
@@ -283,7 +383,7 @@ __device__ __forceinline__ uint32_t bit_of(const uint32_t* __restrict__ bits, in
 
 // contact_tracing.identify_contacts, the find_contacts half (utils.py:131-147):
 // every edge of a stored layer without an index with a traced endpoint marks the
-// other endpoint in its layer's bitmap (dynamic layers: k_trace_dyn)
+// other endpoint in its layer's bitmap (the others: mark_contacts)
 template <int ROUNDS>
 __global__ void __launch_bounds__(EDGE_THREADS) k_trace_scan(covgpu_state st, int t) {
   if (held(st, t)) return;
@@ -302,7 +402,7 @@ __global__ void __launch_bounds__(EDGE_THREADS) k_trace_scan(covgpu_state st, in
   const covgpu_sim_params& sp = st.sims[L->sim];
   const covgpu_testing& T = sp.testing;
   if (!day_active(t, T.trace_start, T.trace_end) || T.thr_trace[L->layer] == 0 || st.trace_count[L->sim] == 0) return;
-  if (L->rp1) return;  // indexed: k_trace_csr visits the traced agents' edges
+  if (L->rp1) return;  // indexed: mark_contacts visits the traced agents' edges
   const int64_t words = (st.n + 31) >> 5;
   uint32_t* contact = st.contact_bits + (int64_t)L->layer * words;
   const int64_t e0 = ((int64_t)blockIdx.x - L->tile_begin) * TILE;
@@ -326,92 +426,20 @@ __global__ void __launch_bounds__(EDGE_THREADS) k_trace_scan(covgpu_state st, in
   }
 }
 
-// find_contacts through the index of each stored layer: a traced agent marks the
-// other endpoint of each of its edges, as p1 and as p2
-__device__ __forceinline__ void trace_csr_block(const covgpu_state& st, int t, const covgpu_agent_block& blk) {
-  const covgpu_sim_params& sp = st.sims[blk.sim];
-  const covgpu_testing& T = sp.testing;
-  if (!day_active(t, T.trace_start, T.trace_end) || st.trace_count[blk.sim] == 0) return;
-  const int64_t i = blk.begin + threadIdx.x;
-  if (i >= blk.end || !((st.trace_bits[i >> 5] >> (i & 31)) & 1u)) return;
-  const int64_t words = (st.n + 31) >> 5;
-  const int64_t local = i - sp.agent_off;
-  for (int l = 0; l < sp.n_layers; ++l) {
-    const int seg = sp.seg_of_layer[l];
-    if (seg < 0 || T.thr_trace[l] == 0) continue;
-    const covgpu_layer& L = st.segments[seg];
-    if (L.dynamic || !L.rp1) continue;
-    uint32_t* contact = st.contact_bits + (int64_t)l * words;
-    for (uint32_t k = L.rp1[local]; k < L.rp1[local + 1]; ++k) {
-      const int32_t b = L.p2[k];
-      atomicOr(contact + (b >> 5), 1u << (b & 31));
-    }
-    for (uint32_t k = L.rp2[local]; k < L.rp2[local + 1]; ++k) {
-      const int32_t a = L.p1[L.perm2[k]];
-      atomicOr(contact + (a >> 5), 1u << (a & 31));
-    }
-  }
-}
-__global__ void __launch_bounds__(AGENT_THREADS) k_trace_csr(covgpu_state st, int t) {
-  if (held(st, t)) return;
-  int64_t b, b_end;
-  if (!agent_range(st, b, b_end)) return;
-  for (; b < b_end; ++b) trace_csr_block(st, t, st.agent_blocks[b]);
-}
-
-// find_contacts over the dynamic layers: one warp per agent block; each traced
-// agent draws its two contact lists (the draws the edge pass makes for that agent
-// as a source) and marks every partner
-constexpr int TRACE_DYN_WARPS = 4;
-__global__ void __launch_bounds__(TRACE_DYN_WARPS * 32) k_trace_dyn(covgpu_state st, int t) {
-  if (held(st, t)) return;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t b = (int64_t)blockIdx.x * TRACE_DYN_WARPS + warp;
-  if (b >= st.n_agent_blocks) return;  // warp-uniform
-  const covgpu_agent_block blk = st.agent_blocks[b];
-  const covgpu_sim_params& sp = st.sims[blk.sim];
-  const covgpu_testing& T = sp.testing;
-  if (!day_active(t, T.trace_start, T.trace_end) || st.trace_count[blk.sim] == 0) return;
-  const int64_t w0 = blk.begin >> 5;  // sims start at multiples of 32
-  const int nw = (int)((blk.end - blk.begin + 31) >> 5);
-  const WarpBits wb = warp_bits_scan(lane < nw ? st.trace_bits[w0 + lane] : 0u);
-  if (wb.total == 0) return;
-  const int64_t words = (st.n + 31) >> 5;
-  const uint32_t n_local = (uint32_t)sp.n_agents, thr = bounded_thr(n_local);
-  const int32_t off = (int32_t)sp.agent_off;
-  for (int l = 0; l < sp.n_layers; ++l) {
-    const int seg = sp.seg_of_layer[l];
-    if (seg < 0 || T.thr_trace[l] == 0 || !st.segments[seg].dynamic) continue;
-    const covgpu_layer& L = st.segments[seg];
-    uint32_t* contact = st.contact_bits + (int64_t)l * words;
-    for (int base = 0; base < wb.total; base += 32) {
-      const int idx = base + lane;
-      int bit;
-      const int wl = warp_bits_nth(wb, nw, idx, bit);
-      if (idx >= wb.total) continue;
-      const uint32_t a = (uint32_t)((w0 + wl) * 32 + bit - off);
-      int k[2];
-      dyn_counts(L.dyn_cdf, L.dyn_k, a, (uint32_t)t, (uint32_t)l, sp.key0, sp.key1, k[0], k[1]);
-      for (int d = 0; d < 2; ++d) {
-        uint4 pw = make_uint4(0u, 0u, 0u, 0u);
-        for (int j = 0; j < k[d]; ++j) {
-          if ((j & 3) == 0) pw = dyn_partner_block(a, d, j, (uint32_t)t, (uint32_t)l, sp.key0, sp.key1);
-          const int32_t g = off + (int32_t)dyn_partner(word_of(pw, j & 3), n_local, thr, a, d, j, (uint32_t)t,
-                                                       (uint32_t)l, sp.key0, sp.key1);
-          atomicOr(contact + (g >> 5), 1u << (g & 31));
-        }
-      }
-    }
-  }
-}
-
 // contact_tracing.notify_contacts (interventions.py:1120-1145) with the
 // binomial_filter of identify_contacts, then update_states_post
 // (people.py:189-196: check_diagnosed, check_quar, check_enter_iso)
-// One agent block of the post pass; the day's diagnoses, quarantines and
-// isolations are counted into the thread's accumulators
+// One agent block of the post pass, its fields already loaded (PostIn); the day's
+// diagnoses, quarantines and isolations are counted into the thread's accumulators
+struct PostIn {
+  uint32_t f;
+  float dpt, dd;   // date_pos_test, date_diagnosed
+  int32_t pq;      // today's pending-quarantine slot
+  uint32_t word;   // lane l: the warp's contact word of layer l, on tracing days
+};
 __device__ __forceinline__ void post_block(const covgpu_state& st, int t, const covgpu_agent_block& blk,
-                                           unsigned& acc_diag, unsigned& acc_quar, unsigned& acc_iso) {
+                                           const PostIn& in, unsigned& acc_diag, unsigned& acc_quar,
+                                           unsigned& acc_iso) {
   const covgpu_sim_params& sp = st.sims[blk.sim];
   const covgpu_testing& T = sp.testing;
   const int64_t i = blk.begin + threadIdx.x;
@@ -419,51 +447,36 @@ __device__ __forceinline__ void post_block(const covgpu_state& st, int t, const 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t words = (st.n + 31) >> 5;
   const int64_t w = (blk.begin + warp * 32) >> 5;
-  const bool warp_in = blk.begin + warp * 32 < blk.end;
   const float tf = (float)t;
   const int R = st.pending_slots;
   unsigned c_diag = 0, c_quar = 0, c_iso = 0;
-  // the agent's fields the checks read, loaded together (one round trip): flags,
-  // date_pos_test, date_diagnosed, today's pending-quarantine slot, date_end_quarantine
   const float nanf_ = __int_as_float(0x7fc00000);
-  uint32_t f = 0u;
-  float a_dpt = nanf_, a_dd = nanf_, a_deq = nanf_;
-  int32_t a_pq = -1;
-  int32_t* pq_today = st.pending_quar + (int64_t)(t % R) * st.n + i;
-  if (valid) {
-    f = st.flags[i];
-    a_dpt = date_row(st, COVGPU_DATE_POS_TEST)[i];
-    a_dd = date_row(st, COVGPU_DATE_DIAGNOSED)[i];
-    a_pq = *pq_today;
-    a_deq = date_row(st, COVGPU_DATE_END_QUARANTINE)[i];
-  }
+  uint32_t f = in.f;
+  const float a_dpt = in.dpt, a_dd = in.dd;
+  int32_t a_pq = in.pq;
   const uint32_t f_in = f;
 
-  // ---- notify the contacts found by the scan (only on tracing days)
-  if (day_active(t, T.trace_start, T.trace_end) && warp_in) {
-    for (int l = 0; l < sp.n_layers; ++l) {
-      uint32_t* cw = st.contact_bits + (int64_t)l * words + w;
-      const uint32_t word = *cw;
-      __syncwarp();
-      if (!word) continue;
-      if (lane == 0) *cw = 0u;  // leave the bitmap clear for the next tracing day
-      if (!valid || !((word >> lane) & 1u)) continue;
-      const uint32_t local = (uint32_t)(i - sp.agent_off);
-      const uint4 u = philox(make_uint4(local, (uint32_t)l, (uint32_t)t, TAG_TRACE), sp.key0, sp.key1);
-      if (!bern52_thr(u.x, u.y, T.thr_trace[l]) || (f & B_DEAD)) continue;
-      f |= B_KCONT;
-      float* dkc = date_row(st, COVGPU_DATE_KNOWN_CONTACT) + i;
-      const float cand = __double2float_rn(__dadd_rn((double)t, T.trace_time[l]));
-      if (isnan(*dkc) || cand < *dkc) *dkc = cand;  // np.fmin
-      const int start = t + T.trace_start_off[l];
-      const int32_t end = start + T.trace_period[l];
-      if (start == t) {  // today's slot: check_quar below reads it from a_pq
-        if (a_pq < 0 || end > a_pq) a_pq = end;
-        continue;
-      }
-      int32_t* pq = st.pending_quar + (int64_t)(start % R) * st.n + i;
-      if (*pq < 0 || end > *pq) *pq = end;  // check_quar keeps the latest end of a day's requests
+  // ---- notify the contacts found on this tracing day, layer by layer
+  for (unsigned layers = __ballot_sync(0xffffffffu, in.word != 0u); layers; layers &= layers - 1) {
+    const int l = __ffs(layers) - 1;
+    const uint32_t word = __shfl_sync(0xffffffffu, in.word, l);
+    if (lane == 0) st.contact_bits[(int64_t)l * words + w] = 0u;  // clear for the next tracing day
+    if (!valid || !((word >> lane) & 1u)) continue;
+    const uint32_t local = (uint32_t)(i - sp.agent_off);
+    const uint4 u = philox(make_uint4(local, (uint32_t)l, (uint32_t)t, TAG_TRACE), sp.key0, sp.key1);
+    if (!bern52_thr(u.x, u.y, T.thr_trace[l]) || (f & B_DEAD)) continue;
+    f |= B_KCONT;
+    float* dkc = date_row(st, COVGPU_DATE_KNOWN_CONTACT) + i;
+    const float cand = __double2float_rn(__dadd_rn((double)t, T.trace_time[l]));
+    if (isnan(*dkc) || cand < *dkc) *dkc = cand;  // np.fmin
+    const int start = t + T.trace_start_off[l];
+    const int32_t end = start + T.trace_period[l];
+    if (start == t) {  // today's slot: check_quar below reads it from a_pq
+      if (a_pq < 0 || end > a_pq) a_pq = end;
+      continue;
     }
+    int32_t* pq = st.pending_quar + (int64_t)(start % R) * st.n + i;
+    if (*pq < 0 || end > *pq) *pq = end;  // check_quar keeps the latest end of a day's requests
   }
 
   if (valid) {
@@ -475,9 +488,12 @@ __device__ __forceinline__ void post_block(const covgpu_state& st, int t, const 
     }
     // ---- check_quar, people.py:335-358
     const int32_t end = a_pq;
+    // only the quarantined, or those asked to be, have an end of quarantine to look at
+    float* p_deq = date_row(st, COVGPU_DATE_END_QUARANTINE) + i;
+    const float a_deq = ((f & B_QUAR) || end >= 0) ? *p_deq : nanf_;
     float deq = a_deq;
     if (end >= 0) {
-      *pq_today = -1;
+      if (in.pq >= 0) st.pending_quar[(int64_t)(t % R) * st.n + i] = -1;
       if (f & B_QUAR) {
         if ((float)end > deq) deq = (float)end;  // max(current, end_day), first argument kept on ties/NaN
       } else if (!(f & (B_DEAD | B_REC | B_DIAG | B_ISO))) {
@@ -488,7 +504,7 @@ __device__ __forceinline__ void post_block(const covgpu_state& st, int t, const 
       }
     }
     if ((f & B_QUAR) && dd == tf) deq = tf;
-    if (__float_as_uint(deq) != __float_as_uint(a_deq)) date_row(st, COVGPU_DATE_END_QUARANTINE)[i] = deq;
+    if (__float_as_uint(deq) != __float_as_uint(a_deq)) *p_deq = deq;
     if ((f & B_QUAR) && defined(deq) && tf >= deq) f &= ~B_QUAR;
     // ---- check_enter_iso, people.py:361-366
     if (dd == tf) {
@@ -527,20 +543,37 @@ __device__ __forceinline__ void post_flush(const covgpu_state& st, int t, int si
   acc_diag = acc_quar = acc_iso = 0;
 }
 
-__global__ void __launch_bounds__(AGENT_THREADS) k_post_pass(covgpu_state st, int t) {
+__global__ void __launch_bounds__(AGENT_THREADS, PASS_BLOCKS) k_post_pass(covgpu_state st, int t) {
+  pdl_wait();
   if (held(st, t)) return;
   int64_t b, b_end;
   if (!agent_range(st, b, b_end)) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t words = (st.n + 31) >> 5;
   int sim = st.agent_blocks[b].sim;
   unsigned acc_diag = 0, acc_quar = 0, acc_iso = 0;
+  const int32_t* pending = st.pending_quar + (int64_t)(t % st.pending_slots) * st.n;
   for (; b < b_end; ++b) {
     const covgpu_agent_block blk = st.agent_blocks[b];
+    const covgpu_sim_params& sp = st.sims[blk.sim];
+    const int64_t i = blk.begin + threadIdx.x, i0 = blk.begin + warp * 32;
+    const float nanf_ = __int_as_float(0x7fc00000);
+    PostIn in{0u, nanf_, nanf_, -1, 0u};
+    if (i < blk.end) {
+      in.f = st.flags[i];
+      in.dpt = date_row(st, COVGPU_DATE_POS_TEST)[i];
+      in.dd = date_row(st, COVGPU_DATE_DIAGNOSED)[i];
+      in.pq = pending[i];
+    }
+    if (lane < sp.n_layers && i0 < blk.end && day_active(t, sp.testing.trace_start, sp.testing.trace_end))
+      in.word = st.contact_bits[(int64_t)lane * words + (i0 >> 5)];
     if (blk.sim != sim) {
       post_flush(st, t, sim, acc_diag, acc_quar, acc_iso);
       sim = blk.sim;
     }
-    post_block(st, t, blk, acc_diag, acc_quar, acc_iso);
+    post_block(st, t, blk, in, acc_diag, acc_quar, acc_iso);
   }
+  pdl_trigger();
   post_flush(st, t, sim, acc_diag, acc_quar, acc_iso);
 }
 
@@ -582,30 +615,35 @@ namespace covgpu {
 
 int launch_test_trace(const covgpu_state* st, int t, cudaStream_t s) {
   if (!st->has_testing) return COVGPU_OK;
-  k_test_prep<<<(unsigned)st->n_sims, 256, 0, s>>>(*st, t);
+  // bit 4: no sim has anything to prepare (no swab delay, capacity or influenza-like illness)
+  if (!(st->has_testing & 16)) k_test_prep<<<(unsigned)st->n_sims, 256, 0, s>>>(*st, t);
   if (st->has_testing & 2) {  // some sim has a swab delay
     static const int64_t hist_wave = wave_blocks(k_swab_hist, AGENT_THREADS);
     k_swab_hist<<<wave_grid(st, hist_wave), AGENT_THREADS, 0, s>>>(*st, t);
   }
-  static const int64_t test_wave = wave_blocks(k_test_pass, AGENT_THREADS);
-  k_test_pass<<<wave_grid(st, test_wave), AGENT_THREADS, 0, s>>>(*st, t);
-  if (st->has_testing & 4) k_trace_cap<<<(unsigned)st->n_sims, 256, 0, s>>>(*st, t);  // a tracing capacity
-  if (st->n_tiles > 0 && !(st->has_testing & 8)) {  // some stored layer is traced without an index
-    const dim3 grid((unsigned)st->n_tiles);
-    switch (st->edge_tile) {
-      case 1024: k_trace_scan<1><<<grid, EDGE_THREADS, 0, s>>>(*st, t); break;
-      case 2048: k_trace_scan<2><<<grid, EDGE_THREADS, 0, s>>>(*st, t); break;
-      case 8192: k_trace_scan<8><<<grid, EDGE_THREADS, 0, s>>>(*st, t); break;
-      default: k_trace_scan<4><<<grid, EDGE_THREADS, 0, s>>>(*st, t); break;
+  const bool scan = st->n_tiles > 0 && !(st->has_testing & 8);  // some stored layer is traced without an index
+  const bool capacity = st->has_testing & 4;
+  if (!scan && !capacity) {
+    static const int64_t mark_wave = wave_blocks(k_test_pass<true>, AGENT_THREADS);
+    launch_pdl(k_test_pass<true>, wave_grid(st, mark_wave), AGENT_THREADS, 0, s, *st, t);
+  } else {
+    static const int64_t test_wave = wave_blocks(k_test_pass<false>, AGENT_THREADS);
+    launch_pdl(k_test_pass<false>, wave_grid(st, test_wave), AGENT_THREADS, 0, s, *st, t);
+    if (capacity) k_trace_cap<<<(unsigned)st->n_sims, 256, 0, s>>>(*st, t);
+    if (scan) {
+      const dim3 grid((unsigned)st->n_tiles);
+      switch (st->edge_tile) {
+        case 1024: k_trace_scan<1><<<grid, EDGE_THREADS, 0, s>>>(*st, t); break;
+        case 2048: k_trace_scan<2><<<grid, EDGE_THREADS, 0, s>>>(*st, t); break;
+        case 8192: k_trace_scan<8><<<grid, EDGE_THREADS, 0, s>>>(*st, t); break;
+        default: k_trace_scan<4><<<grid, EDGE_THREADS, 0, s>>>(*st, t); break;
+      }
     }
+    static const int64_t marks_wave = wave_blocks(k_trace_marks, AGENT_THREADS);
+    k_trace_marks<<<wave_grid(st, marks_wave), AGENT_THREADS, 0, s>>>(*st, t);
   }
-  static const int64_t csr_wave = wave_blocks(k_trace_csr, AGENT_THREADS);
-  k_trace_csr<<<wave_grid(st, csr_wave), AGENT_THREADS, 0, s>>>(*st, t);
-  if (st->n_dynamic)
-    k_trace_dyn<<<(unsigned)((st->n_agent_blocks + TRACE_DYN_WARPS - 1) / TRACE_DYN_WARPS), TRACE_DYN_WARPS * 32, 0,
-                  s>>>(*st, t);
   static const int64_t post_wave = wave_blocks(k_post_pass, AGENT_THREADS);
-  k_post_pass<<<wave_grid(st, post_wave), AGENT_THREADS, 0, s>>>(*st, t);
+  launch_pdl(k_post_pass, wave_grid(st, post_wave), AGENT_THREADS, 0, s, *st, t);
   return launch_status();
 }
 

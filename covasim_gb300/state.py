@@ -354,6 +354,8 @@ class BatchState:
                             for sp in self.specs)
         self.has_capacity = any((sp.testing or {}).get('trace') and sp.testing['trace'].get('capacity') is not None
                                 for sp in self.specs)
+        self.has_ili = any((sp.testing or {}).get('test') and sp.testing['test'].get('ili_prev') is not None
+                           for sp in self.specs)
         self.pending_slots = 1
         self.n_contact_layers = max(len(sp.layers) for sp in self.specs) or 1
         if self.has_testing:
@@ -922,7 +924,8 @@ class BatchState:
         st.has_testing = 0
         if self.has_testing:  # bit 0 and its refinements
             st.has_testing = (1 | (2 if self.has_swab else 0) | (4 if self.has_capacity else 0) |
-                              (8 if all(rec.dynamic or rec.rp1 for rec in self.segments) else 0))
+                              (8 if all(rec.dynamic or rec.rp1 for rec in self.segments) else 0) |
+                              (0 if self.has_swab or self.has_capacity or self.has_ili else 16))
         st.pending_slots = self.pending_slots
         st.n_contact_layers = self.n_contact_layers
         if self.has_testing:
