@@ -25,6 +25,7 @@ N_RES_F = 3
 FX_NAB_BITS = 24
 FX_IMM_BITS = 32
 NO_VARIANT = 0xFF
+WALK_ALL = -2  # covgpu_state.src_walk: every stored layer walked every day (COVGPU_WALK_ALL)
 NOALLOC_MAX_EDGES = 1 << 24   # covgpu_infections_noalloc limit (COVGPU_NOALLOC_MAX_EDGES)
 NO_SUBTARGET = 0xFFFFFFFFFFFFFFFF  # covgpu_testing.sub_thr: no subtarget (COVGPU_NO_SUBTARGET)
 EDGE_TILE = '2048w'       # default edge pass: 2048-edge tiles, the stored layers' pass as one wave of blocks
@@ -109,7 +110,7 @@ class Layer(C.Structure):
                 ('tile_begin', C.c_int64), ('sim', C.c_int32), ('layer', C.c_int32), ('dynamic', C.c_int32),
                 ('beta_const', C.c_float), ('iso_factor', C.c_float), ('quar_factor', C.c_float),
                 ('dyn_k', C.c_int32), ('rp1', C.c_void_p), ('rp2', C.c_void_p), ('perm2', C.c_void_p),
-                ('dyn_cdf', C.c_void_p), ('dyn_rse_max', C.c_float), ('_pad2', C.c_int32)]
+                ('dyn_cdf', C.c_void_p), ('dyn_rse_max', C.c_float), ('_pad2', C.c_int32), ('rev1', C.c_void_p)]
 
 
 class AgentBlock(C.Structure):
@@ -203,6 +204,8 @@ def lib():
         L.covgpu_trace_index_scratch.restype = i64
         L.covgpu_trace_index.argtypes = [vp, vp, i64, i64, i64, vp, vp, vp, vp, vp]
         L.covgpu_trace_index.restype = C.c_int
+        L.covgpu_agent_index.argtypes = [vp, vp, i64, i64, i64, vp, vp, vp, vp, vp, vp]
+        L.covgpu_agent_index.restype = C.c_int
         L.covgpu_pop_scan_scratch.argtypes = [i64]
         L.covgpu_pop_scan_scratch.restype = i64
         f64 = C.c_double
@@ -256,6 +259,6 @@ EXPORTED = ['covgpu_version', 'covgpu_abi_layout', 'covgpu_viral_load', 'covgpu_
             'covgpu_infections', 'covgpu_infections_find', 'covgpu_infections_emit',
             'covgpu_infections_noalloc', 'covgpu_agent_step', 'covgpu_edge_pass', 'covgpu_infect_claims',
             'covgpu_infect_list', 'covgpu_import_day', 'covgpu_rescale_check', 'covgpu_layer_lists', 'covgpu_run_days', 'covgpu_test_trace',
-            'covgpu_lik_targets', 'covgpu_trace_index_scratch', 'covgpu_trace_index', 'covgpu_edge_resident_bytes',
+            'covgpu_lik_targets', 'covgpu_trace_index_scratch', 'covgpu_trace_index', 'covgpu_agent_index', 'covgpu_edge_resident_bytes',
             'covgpu_check', 'covgpu_check_immunity', 'covgpu_update_nab', 'covgpu_update_peak_nab',
             'covgpu_pop_scan_scratch'] + POP_FUNCS

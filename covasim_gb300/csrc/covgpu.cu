@@ -12,10 +12,10 @@
 //       128-bit reads, source->target candidates queued per warp in shared memory,
 //       then compute_trans_sus folded in lane-packed, Philox Bernoullis,
 //       warp-ballot compaction of events, atomicMin first-infector claim;
-//   k_dyn_pass       the redrawn layers (base.py:1849-1876): the day's sources'
+//   k_source_pass    the redrawn layers (base.py:1849-1876): the day's sources'
 //       contact lists drawn from Philox and thinned, the same candidates' path;
-//       on quiet days its second half of blocks walks the stored layers from the
-//       sources instead of the tile pass (k_src_pass: the walk on its own);
+//       and the stored layers walked from the sources through their agent index
+//       instead of the tile pass, in alternating blocks of one launch;
 //   k_infect_claims / k_infect_list   People.infect (people.py:435-586) +
 //       update_peak_nab (immunity.py:138-202).
 // The reference's standalone numba functions are in covgpu_reference.cu, the
@@ -50,11 +50,7 @@ namespace {
 #define AGENT_BOUNDS __launch_bounds__(AGENT_THREADS)
 #endif
 constexpr int EQ_ROUND = 32 * EDGE_VEC;  // most candidates one warp appends per round (one per edge)
-#ifndef COVGPU_EQ_CAP
-#define COVGPU_EQ_CAP 256
-#endif
-constexpr int EQ_CAP = COVGPU_EQ_CAP;  // candidate queue entries per warp (drained when a round could overflow);
-                                       // 192 and 160, which leave L1 more room, measured slower
+constexpr int EQ_CAP = 32 + EQ_ROUND;  // candidate queue entries per warp: fewer than 32 left over + one round
 static_assert(2 * EDGE_TILE_MAX <= 65536, "queue entries pack (edge within the tile, direction) in 16 bits");
 constexpr int CALL_TAG_SEED = 1;       // covgpu_infect_list call_tag of the day-0 seed infections
 constexpr int CALL_TAG_IMPORT = 2;     // the daily importations (variant importations: 2 + variant)
@@ -671,24 +667,35 @@ __device__ __forceinline__ void queue_push(EdgeQueue& q, int& qn, bool has, int3
   qn += __popc(mask);
 }
 
-// phase B: one candidate per lane, then the warp-aggregated event append
-// (LIK: with the likelihood terms)
+// phase B of the queue's entries [base, base + 32) (those below qn): one candidate per
+// lane, then the warp-aggregated event append (LIK: with the likelihood terms)
 template <bool LIK>
 __device__ __forceinline__ void queue_drain(const covgpu_state& st, const SegCtx& c, int t, int64_t e0,
-                                            EdgeQueue& q, int qn, LikAcc& acc) {
+                                            EdgeQueue& q, int base, int qn, LikAcc& acc) {
+  const int i = base + (threadIdx.x & 31);
+  bool hit = false;
+  uint32_t v = 0;
+  int32_t s = 0, g = 0;
+  uint32_t m = 0;
+  if (i < qn) {
+    s = q.s[i]; g = q.g[i]; m = q.m[i];
+    hit = edge_try<LIK>(st, c, t, e0 + (m >> 1), (int)(m & 1u), s, g, v, acc);
+  }
+  emit(st, hit, hit ? event_key(t, v, c.layer, (int)(m & 1u), e0 + (m >> 1)) : 0ull, g, s);
+}
+// after a round's pushes: full warps from the top of the queue (the order does not
+// matter), fewer than 32 entries stay for the next round; all: those too
+template <bool LIK>
+__device__ __forceinline__ void queue_settle(const covgpu_state& st, const SegCtx& c, int t, int64_t e0,
+                                             EdgeQueue& q, int& qn, bool all, LikAcc& acc) {
   __syncwarp();
-  const int lane = threadIdx.x & 31;
-  for (int base = 0; base < qn; base += 32) {
-    const int i = base + lane;
-    bool hit = false;
-    uint32_t v = 0;
-    int32_t s = 0, g = 0;
-    uint32_t m = 0;
-    if (i < qn) {
-      s = q.s[i]; g = q.g[i]; m = q.m[i];
-      hit = edge_try<LIK>(st, c, t, e0 + (m >> 1), (int)(m & 1u), s, g, v, acc);
-    }
-    emit(st, hit, hit ? event_key(t, v, c.layer, (int)(m & 1u), e0 + (m >> 1)) : 0ull, g, s);
+  while (qn >= 32) {
+    qn -= 32;
+    queue_drain<LIK>(st, c, t, e0, q, qn, qn + 32, acc);
+  }
+  if (all && qn > 0) {
+    queue_drain<LIK>(st, c, t, e0, q, 0, qn, acc);
+    qn = 0;
   }
   __syncwarp();
 }
@@ -823,12 +830,8 @@ __device__ __forceinline__ void edge_tile(const covgpu_state& st, int t, int seg
     const int4 pa = na, pb = nb;
     if (r + 1 < ROUNDS) fetch(r + 1, na, nb);
     edge_round<RES>(st, s_src, pa, pb, eb, e1, e0, q, qn);
-    if (qn > EQ_CAP - EQ_ROUND) {
-      queue_drain<LIK>(st, c, t, e0, q, qn, acc);
-      qn = 0;
-    }
+    queue_settle<LIK>(st, c, t, e0, q, qn, r + 1 == ROUNDS, acc);
   }
-  if (qn > 0) queue_drain<LIK>(st, c, t, e0, q, qn, acc);
 }
 
 // Tiles [k_lo, k_hi) of one stored segment (L, its sim's constants sp) as one
@@ -867,21 +870,14 @@ __device__ __forceinline__ void edge_span(const covgpu_state& st, int t, int seg
   fetch(e_lo, na, nb);
   for (int64_t rb = e_lo; rb < e_hi; rb += ROUND) {
     if (rb + ROUND - e0 > SPAN) {
-      if (qn > 0) {
-        queue_drain<LIK>(st, c, t, e0, q, qn, acc);
-        qn = 0;
-      }
+      queue_settle<LIK>(st, c, t, e0, q, qn, true, acc);
       e0 = rb;
     }
     const int4 pa = na, pb = nb;
     if (rb + ROUND < e_hi) fetch(rb + ROUND, na, nb);
     edge_round<false>(st, nullptr, pa, pb, rb + (int64_t)threadIdx.x * EDGE_VEC, e_hi, e0, q, qn);
-    if (qn > EQ_CAP - EQ_ROUND) {
-      queue_drain<LIK>(st, c, t, e0, q, qn, acc);
-      qn = 0;
-    }
+    queue_settle<LIK>(st, c, t, e0, q, qn, rb + ROUND >= e_hi, acc);
   }
-  if (qn > 0) queue_drain<LIK>(st, c, t, e0, q, qn, acc);
 }
 
 // the likelihood sums of one warp for one (sim, layer), then reset
@@ -1071,15 +1067,20 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_edge_pass_res(covgpu_state s
 // day's sources, not the layer's edges: a quiet day costs a read of the source
 // bitmap.
 constexpr int DYN_WARPS = 8;  // warps per thread block
-// Warps per agent block of the per-source passes (SPLIT, a template parameter: each
-// warp takes 8 / SPLIT of the agent block's eight source-bitmap words). One warp
-// per agent block ran a 1M-agent run 2.7% faster than two (16.8 against 17.26 ms):
-// half the warps to launch and scan on the quiet days, when the pass is all
-// scanning; a state of fewer agent blocks than SPLIT_ONE_MIN keeps two, for the
-// parallelism of its busy days.
+// Warps per agent block of the per-source passes (split: each warp takes 8 / split
+// of the agent block's eight source-bitmap words): one from SPLIT_TARGET agent
+// blocks up, else doubled until that many warps. A warp's set-up is a chain of
+// about six dependent loads, so more warps only pay where the chip would idle: the
+// 1M-agent run took 15.9 ms with one, 16.5 with two, 17.7 with four and 20.0 with
+// eight; 300,000 agents 7.0 ms with two (7.2 with one), 7.3 with four, 7.6 with
+// eight; 100,000 agents the same (8.1 ms) with four and eight.
 constexpr int AB_WORDS = AGENT_THREADS / 32;  // source-bitmap words of an agent block
-constexpr int64_t SPLIT_ONE_MIN = 2048;
-inline int source_split(const covgpu_state* st) { return st->n_agent_blocks >= SPLIT_ONE_MIN ? 1 : 2; }
+constexpr int64_t SPLIT_TARGET = 2048;
+inline int source_split(const covgpu_state* st) {
+  int split = 1;
+  while (split < AB_WORDS && st->n_agent_blocks * split < SPLIT_TARGET) split *= 2;
+  return split;
+}
 
 // the segment constants of dynamic layer segment seg for day t
 __device__ __forceinline__ void dyn_ctx(const covgpu_state& st, const covgpu_sim_params& sp, int seg, int t, SegCtx& c) {
@@ -1125,40 +1126,37 @@ __device__ __forceinline__ int dyn_shift(const covgpu_state& st, const SegCtx& c
 // warp-aggregated event append
 template <bool LIK>
 __device__ __forceinline__ void dyn_drain(const covgpu_state& st, const SegCtx& c, int t, int64_t agent_off,
-                                          EdgeQueue& q, int qn, LikAcc& acc) {
-  __syncwarp();
-  const int lane = threadIdx.x & 31;
-  for (int base = 0; base < qn; base += 32) {
-    const int i = base + lane;
-    bool hit = false;
-    uint32_t v = 0, m = 0;
-    int32_t s = 0, g = 0;
-    uint64_t e = 0;
-    if (i < qn) {
-      s = q.s[i]; g = q.g[i]; m = q.m[i];
-      e = dyn_edge_id((uint32_t)(s - agent_off), m >> 2, (uint32_t)t, (uint32_t)c.layer);
-      hit = edge_try<LIK, false, true>(st, c, t, (int64_t)e, (int)(m & 1u), s, g, v, acc, (m >> 1) & 1u);
-    }
-    emit(st, hit, hit ? event_key(t, v, c.layer, (int)(m & 1u), (int64_t)e) : 0ull, g, s);
+                                          EdgeQueue& q, int base, int qn, LikAcc& acc) {
+  const int i = base + (threadIdx.x & 31);
+  bool hit = false;
+  uint32_t v = 0, m = 0;
+  int32_t s = 0, g = 0;
+  uint64_t e = 0;
+  if (i < qn) {
+    s = q.s[i]; g = q.g[i]; m = q.m[i];
+    e = dyn_edge_id((uint32_t)(s - agent_off), m >> 2, (uint32_t)t, (uint32_t)c.layer);
+    hit = edge_try<LIK, false, true>(st, c, t, (int64_t)e, (int)(m & 1u), s, g, v, acc, (m >> 1) & 1u);
   }
-  __syncwarp();
+  emit(st, hit, hit ? event_key(t, v, c.layer, (int)(m & 1u), (int64_t)e) : 0ull, g, s);
 }
 
 // The redrawn layers of the day's sources for one block's worth (vblock) of
-// agent blocks: SPLIT warps per agent block, each on AB_WORDS / SPLIT source-bitmap words.
-template <bool LIK, int SPLIT>
-__device__ __forceinline__ void dyn_body(const covgpu_state& st, int t, int64_t vblock, EdgeQueue* s_q) {
-  constexpr int DYN_WORDS = AB_WORDS / SPLIT;
+// agent blocks: split warps per agent block, each on AB_WORDS / split source-bitmap words.
+template <bool LIK>
+__device__ __forceinline__ void dyn_body(const covgpu_state& st, int t, int64_t vblock, int split, EdgeQueue* s_q) {
+  const int words = AB_WORDS / split;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t gw = vblock * DYN_WARPS + warp;
-  const int64_t b = gw / SPLIT;  // SPLIT warps per agent block
+  const int64_t b = gw / split;  // split warps per agent block
   if (b >= st.n_agent_blocks) return;  // warp-uniform
   const covgpu_agent_block blk = st.agent_blocks[b];
-  const int w_lo = (int)(gw % SPLIT) * DYN_WORDS;
+  const int w_lo = (int)(gw % split) * words;
   const int nwb = (int)((blk.end - blk.begin + 31) >> 5);
   if (w_lo >= nwb) return;
-  const int nw = min(DYN_WORDS, nwb - w_lo);
+  const int nw = min(words, nwb - w_lo);
   const int64_t w0 = (blk.begin >> 5) + w_lo;  // sims start at multiples of 32
+  pdl_wait();
+  if (held(st, t)) return;
   const WarpBits wb = warp_bits_scan(lane < nw ? __ldg(st.roles + w0 + lane) : 0u);
   if (wb.total == 0) return;
   const covgpu_sim_params& sp = st.sims[blk.sim];
@@ -1238,108 +1236,144 @@ __device__ __forceinline__ void dyn_body(const covgpu_state& st, int t, int64_t 
         for (int r4 = 0; r4 < 4; ++r4)
           queue_push(q, qn, (tb >> r4) & 1u, os, g[r4],
                      ((uint32_t)(je + r4) << 2) | (((pm >> r4) & 1u) << 1) | (uint32_t)d);
-        if (qn > EQ_CAP - 4 * 32) {
-          dyn_drain<LIK>(st, c, t, sp.agent_off, q, qn, acc);
-          qn = 0;
+        __syncwarp();
+        while (qn >= 32) {  // full warps from the top of the queue
+          qn -= 32;
+          dyn_drain<LIK>(st, c, t, sp.agent_off, q, qn, qn + 32, acc);
         }
+        __syncwarp();
       }
     }
-    if (qn > 0) dyn_drain<LIK>(st, c, t, sp.agent_off, q, qn, acc);
+    if (qn > 0) dyn_drain<LIK>(st, c, t, sp.agent_off, q, 0, qn, acc);
     if (LIK) lik_flush_warp(st, t, blk.sim, l, acc);
+    __syncwarp();  // the queue is read before the next layer fills it
   }
 }
 
 // The walk of the stored layers from the day's sources (seg_walked): the warps and
-// source-bitmap words of the redrawn layers' pass. For each indexed stored
-// layer the warp's sources' edges (as p1: [rp1[a], rp1[a + 1]); as p2: the edges
-// perm2[rp2[a] .. rp2[a + 1])) are flattened across the lanes 32 at a time, each
-// lane finding its source by a search over the lanes' prefix counts; an edge whose
-// other endpoint is a target is queued with its index and direction (1: the
-// source is p2, as in the tile pass) and drained through edge_try.
+// source-bitmap words of the redrawn layers' pass. Each (source, walked layer) of a
+// warp is an item; 32 items at a time, their edges (as p1: [rp1[a], rp1[a + 1]); as
+// p2: entries rp2[a] .. rp2[a + 1] of perm2, the edge, and rev1, its p1) are
+// flattened across the lanes, each lane finding its item by a search over the
+// lanes' prefix counts, WALK_U * 32 edges in flight at a time. An edge whose other
+// endpoint is a target is queued with its index, layer and direction (1: the
+// source is p2, as in the tile pass), and the queue drains through edge_try 32
+// candidates at a time, whatever their layers (the likelihood's sums are kept per
+// layer, so its walk takes one layer after another). It waits on memory: at the
+// peak of a 1M-agent hybrid epidemic (about a quarter infectious) 98 us, against
+// 57 us for the tile pass, whose reads are streams; below a tenth infectious it is
+// the cheaper one, and in a launch with the redrawn layers' draws at every size
+// up to some hundred thousand agents.
 constexpr int SRC_WARPS = 8;
-struct SrcQueue {
-  int32_t s[EQ_CAP];   // source agent
-  int32_t g[EQ_CAP];   // target agent | direction << 31
-  uint32_t e[EQ_CAP];  // edge index in the layer
+constexpr int WALK_U = 2;  // 1 and 4 within 1% (4 slower)
+constexpr int WQ_CAP = 32 + 32 * WALK_U;  // fewer than 32 left over + one round's pushes
+struct WalkQueue {
+  int32_t s[WQ_CAP];   // source agent
+  int32_t g[WQ_CAP];   // target agent | direction << 31
+  uint32_t e[WQ_CAP];  // edge index in the layer
+  uint8_t l[WQ_CAP];   // walked layer (index into the warp's WalkLayer copies)
+};
+struct WalkLayer {  // a walked layer's record with the day's beta_layer
+  const uint32_t *rp1, *rp2, *perm2;
+  const int32_t *p1, *p2, *rev1;
+  const float* beta;
+  int64_t n_edges;
+  float beta_const, beta_layer, quar_factor, iso_factor;
+  int32_t layer, seg;
+};
+struct WalkShared {
+  WalkQueue q;
+  WalkLayer l[COVGPU_MAX_LAYERS];
 };
 
-__device__ __forceinline__ void src_push(SrcQueue& q, int& qn, bool has, int32_t s, int32_t gd, uint32_t e) {
-  const unsigned mask = __ballot_sync(0xffffffffu, has);
-  if (has) {
-    const int pos = qn + __popc(mask & ((1u << (threadIdx.x & 31)) - 1u));
-    q.s[pos] = s; q.g[pos] = gd; q.e[pos] = e;
+// the queue's entries [base, base + 32) (those below qn), one candidate per lane
+template <bool LIK>
+__device__ __forceinline__ void walk_drain(const covgpu_state& st, SegCtx& c, int t, const WalkShared& w, int base,
+                                           int qn, LikAcc& acc) {
+  const int i = base + (threadIdx.x & 31);
+  bool hit = false;
+  uint32_t v = 0;
+  int32_t s = 0, g = 0;
+  int d = 0;
+  int64_t e = 0;
+  if (i < qn) {
+    s = w.q.s[i];
+    const uint32_t gd = (uint32_t)w.q.g[i];
+    g = (int32_t)(gd & 0x7FFFFFFFu);
+    d = (int)(gd >> 31);
+    e = (int64_t)w.q.e[i];
+    const WalkLayer& L = w.l[w.q.l[i]];
+    c.seg = L.seg;
+    c.layer = L.layer;
+    c.n_edges = L.n_edges;
+    c.edge_beta = L.beta;
+    c.beta_const = L.beta_const;
+    c.beta_layer = L.beta_layer;
+    c.quar_factor = L.quar_factor;
+    c.iso_factor = L.iso_factor;
+    hit = edge_try<LIK>(st, c, t, e, d, s, g, v, acc);
   }
-  qn += __popc(mask);
+  emit(st, hit, hit ? event_key(t, v, c.layer, d, e) : 0ull, g, s);
 }
 
 template <bool LIK>
-__device__ __forceinline__ void src_drain(const covgpu_state& st, const SegCtx& c, int t, SrcQueue& q, int qn,
-                                          LikAcc& acc) {
-  __syncwarp();
-  const int lane = threadIdx.x & 31;
-  for (int base = 0; base < qn; base += 32) {
-    const int i = base + lane;
-    bool hit = false;
-    uint32_t v = 0;
-    int32_t s = 0, g = 0;
-    int d = 0;
-    int64_t e = 0;
-    if (i < qn) {
-      s = q.s[i];
-      const uint32_t gd = (uint32_t)q.g[i];
-      g = (int32_t)(gd & 0x7FFFFFFFu);
-      d = (int)(gd >> 31);
-      e = (int64_t)q.e[i];
-      hit = edge_try<LIK>(st, c, t, e, d, s, g, v, acc);
-    }
-    emit(st, hit, hit ? event_key(t, v, c.layer, d, e) : 0ull, g, s);
-  }
-  __syncwarp();
-}
-
-template <bool LIK, int SPLIT>
-__device__ __forceinline__ void src_body(const covgpu_state& st, int t, int64_t vblock, SrcQueue* s_q) {
-  constexpr int DYN_WORDS = AB_WORDS / SPLIT;
+__device__ __forceinline__ void walk_body(const covgpu_state& st, int t, int64_t vblock, int split, WalkShared* s_w) {
+  const int words = AB_WORDS / split;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t gw = vblock * SRC_WARPS + warp;
-  const int64_t b = gw / SPLIT;  // SPLIT warps per agent block
+  const int64_t b = gw / split;  // split warps per agent block
   if (b >= st.n_agent_blocks) return;  // warp-uniform
   const covgpu_agent_block blk = st.agent_blocks[b];
-  const covgpu_sim_params& sp = st.sims[blk.sim];
-  int first = -1;  // the sim's first walked layer
-  for (int l = 0; l < sp.n_layers && first < 0; ++l) {
-    const int seg = sp.seg_of_layer[l];
-    if (seg >= 0 && seg_walked(st, st.segments[seg], t)) first = l;
-  }
-  if (first < 0) return;
-  const int w_lo = (int)(gw % SPLIT) * DYN_WORDS;
+  const int w_lo = (int)(gw % split) * words;
   const int nwb = (int)((blk.end - blk.begin + 31) >> 5);
   if (w_lo >= nwb) return;
-  const int nw = min(DYN_WORDS, nwb - w_lo);
+  const int nw = min(words, nwb - w_lo);
   const int64_t w0 = (blk.begin >> 5) + w_lo;  // sims start at multiples of 32
+  // the layers' records are read-only: copied before the wait
+  const covgpu_sim_params& sp = st.sims[blk.sim];
+  WalkShared& w = s_w[warp];
+  const int seg = lane < sp.n_layers ? sp.seg_of_layer[lane] : -1;
+  bool walked = false;
+  if (seg >= 0) {
+    const covgpu_layer& L = st.segments[seg];
+    walked = !L.dynamic && L.rp1;
+    if (walked)
+      w.l[lane] = WalkLayer{L.rp1, L.rp2, L.perm2, L.p1, L.p2, L.rev1, L.beta, L.n_edges, L.beta_const, 0.0f,
+                            L.quar_factor, L.iso_factor, lane, seg};
+  }
+  pdl_wait();
+  if (held(st, t)) return;
   const WarpBits wb = warp_bits_scan(lane < nw ? __ldg(st.roles + w0 + lane) : 0u);
   if (wb.total == 0) return;
+  walked = walked && seg_walked(st, st.segments[seg], t);
+  const unsigned mask = __ballot_sync(0xffffffffu, walked);  // the walked layers
+  if (!mask) return;
+  if (walked) w.l[lane].beta_layer = sp.beta_layer_tab[(int64_t)t * sp.n_layers + lane];
+  __syncwarp();
+  SegCtx c;
+  c.L = nullptr;
+  c.rse_max = 0.0f;
+  c.asymp_factor = sp.asymp_factor;
+  c.nv = sp.n_variants;
+  c.key0 = sp.key0;
+  c.key1 = sp.key1;
+  c.beta_t = sp.beta_tab + (int64_t)t * c.nv;
+  c.sim = blk.sim;
   const int32_t off = (int32_t)sp.agent_off;
-  SrcQueue& q = s_q[warp];
+  const int nwl = __popc(mask);
+  const int layer_k = lane < nwl ? nth_bit(mask, lane) : 0;  // lane k: the k-th walked layer
   LikAcc acc;
-  for (int l = first; l < sp.n_layers; ++l) {
-    const int seg = sp.seg_of_layer[l];
-    if (seg < 0) continue;
-    const covgpu_layer& L = st.segments[seg];
-    if (!seg_walked(st, L, t)) continue;
-    SegCtx c;
-    dyn_ctx(st, sp, seg, t, c);
-    c.edge_beta = L.beta;
-    const int32_t* p1 = L.p1;
-    const int32_t* p2 = L.p2;
+  for (int l0 = 0; l0 < nwl; l0 += LIK ? 1 : nwl) {
+    const int nl = LIK ? 1 : nwl, items = wb.total * nl;
     int qn = 0;
-    for (int base = 0; base < wb.total; base += 32) {
-      const int idx = base + lane;
+    for (int base = 0; base < items; base += 32) {
+      const int idx = base + lane, src = idx / nl, li = __shfl_sync(0xffffffffu, layer_k, l0 + idx - src * nl);
       int bit;
-      const int wl = warp_bits_nth(wb, nw, idx, bit);
+      const int wl = warp_bits_nth(wb, nw, src, bit);
       const int32_t s = (int32_t)((w0 + wl) * 32 + bit);
       uint32_t k1 = 0, n1 = 0, k2 = 0, n = 0;
-      if (idx < wb.total) {
+      if (idx < items) {
+        const WalkLayer& L = w.l[li];
         const uint32_t a = (uint32_t)(s - off);
         k1 = __ldg(L.rp1 + a);
         n1 = __ldg(L.rp1 + a + 1) - k1;
@@ -1352,109 +1386,111 @@ __device__ __forceinline__ void src_body(const covgpu_state& st, int t, int64_t 
         const uint32_t y = __shfl_up_sync(0xffffffffu, pre, o);
         if (lane >= o) pre += y;
       }
-      const uint32_t total = __shfl_sync(0xffffffffu, pre, 31);
-      for (uint32_t j0 = 0; j0 < total; j0 += 32) {
-        const uint32_t j = j0 + (uint32_t)lane;
-        int owner = 0;  // the first lane whose inclusive prefix exceeds j
+      const uint32_t total = __shfl_sync(0xffffffffu, pre, 31), beg = pre - n;
+      const uint32_t k2r = k2 - n1 - beg, k1r = k1 - beg;  // entry j is edge k1r + j, or entry k2r + j of perm2
+      const uint32_t mid = beg + n1;                       // the first of the latter
+      for (uint32_t j0 = 0; j0 < total; j0 += 32 * WALK_U) {
+        int32_t os[WALK_U], g[WALK_U];
+        uint32_t e[WALK_U], dl[WALK_U];
 #pragma unroll
-        for (int step = 16; step > 0; step >>= 1)
-          if (__shfl_sync(0xffffffffu, pre, owner + step - 1) <= j) owner += step;
-        owner = min(owner, 31);
-        const int32_t os = __shfl_sync(0xffffffffu, s, owner);
-        const uint32_t ok1 = __shfl_sync(0xffffffffu, k1, owner), on1 = __shfl_sync(0xffffffffu, n1, owner);
-        const uint32_t ok2 = __shfl_sync(0xffffffffu, k2, owner);
-        const uint32_t obeg = __shfl_sync(0xffffffffu, pre - n, owner);
-        bool has = false;
-        int32_t g = 0;
-        uint32_t e = 0, d = 0;
-        if (j < total) {
-          const uint32_t r = j - obeg;
-          if (r < on1) {
-            e = ok1 + r;
-            g = __ldg(p2 + e);
-          } else {
-            e = __ldg(L.perm2 + ok2 + (r - on1));
-            g = __ldg(p1 + e);
-            d = 1u;
+        for (int u = 0; u < WALK_U; ++u) {
+          const uint32_t j = j0 + 32u * u + (uint32_t)lane;
+          int owner = 0;  // the first lane whose inclusive prefix exceeds j
+#pragma unroll
+          for (int step = 16; step > 0; step >>= 1)
+            if (__shfl_sync(0xffffffffu, pre, owner + step - 1) <= j) owner += step;
+          owner = min(owner, 31);
+          os[u] = __shfl_sync(0xffffffffu, s, owner);
+          const uint32_t ok1 = __shfl_sync(0xffffffffu, k1r, owner), ok2 = __shfl_sync(0xffffffffu, k2r, owner);
+          const uint32_t omid = __shfl_sync(0xffffffffu, mid, owner);
+          const int oli = __shfl_sync(0xffffffffu, li, owner);
+          g[u] = -1;
+          e[u] = 0;
+          dl[u] = (uint32_t)oli;
+          if (j < total) {
+            const WalkLayer& L = w.l[oli];
+            if (j < omid) {
+              e[u] = ok1 + j;
+              g[u] = __ldg(L.p2 + e[u]);
+            } else {
+              e[u] = __ldg(L.perm2 + (ok2 + j));
+              g[u] = L.rev1 ? __ldg(L.rev1 + (ok2 + j)) : __ldg(L.p1 + e[u]);
+              dl[u] |= 0x80000000u;
+            }
           }
-          has = tgt_bit(st, g) != 0u;
         }
-        src_push(q, qn, has, os, (int32_t)((uint32_t)g | (d << 31)), e);
-        if (qn > EQ_CAP - 32) {
-          src_drain<LIK>(st, c, t, q, qn, acc);
-          qn = 0;
+        bool has[WALK_U];
+#pragma unroll
+        for (int u = 0; u < WALK_U; ++u) has[u] = g[u] >= 0 && tgt_bit(st, g[u]) != 0u;
+#pragma unroll
+        for (int u = 0; u < WALK_U; ++u) {
+          const unsigned m = __ballot_sync(0xffffffffu, has[u]);
+          if (has[u]) {
+            const int pos = qn + __popc(m & ((1u << lane) - 1u));
+            w.q.s[pos] = os[u];
+            w.q.g[pos] = (int32_t)((uint32_t)g[u] | (dl[u] & 0x80000000u));
+            w.q.e[pos] = e[u];
+            w.q.l[pos] = (uint8_t)dl[u];
+          }
+          qn += __popc(m);
         }
+        __syncwarp();
+        while (qn >= 32) {  // full warps from the top of the queue (the order does not matter)
+          qn -= 32;
+          walk_drain<LIK>(st, c, t, w, qn, qn + 32, acc);
+        }
+        __syncwarp();
       }
     }
-    if (qn > 0) src_drain<LIK>(st, c, t, q, qn, acc);
-    if (LIK) lik_flush_warp(st, t, blk.sim, l, acc);
+    if (qn > 0) walk_drain<LIK>(st, c, t, w, 0, qn, acc);
+    if (LIK) lik_flush_warp(st, t, blk.sim, __shfl_sync(0xffffffffu, layer_k, l0), acc);
+    __syncwarp();
   }
 }
 
+static_assert(EQ_CAP >= 31 + 4 * 32, "one round of dyn_body");
 static_assert(SRC_WARPS == DYN_WARPS, "the per-source passes share their launch shape");
 
-// The redrawn layers' pass (dyn_body), and with WALK also the walk of the stored
-// layers from the day's sources (src_body) in blocks [dyn_blocks, 2 dyn_blocks)
-// of the same launch: both start from the day's source bitmap, so on the days the
-// stored layers are walked the walk runs beside the redrawn layers' draws instead
-// of after the stored layers' (then empty) tile pass. Four resident blocks per SM
-// (64 registers): the redrawn layers' pass over a 100-day 1M-agent run took
+// The per-source passes: the redrawn layers' (DYN), the walk of the stored layers
+// (WALK), or both in one launch, alternating blocks of the two (they start from the
+// day's source bitmap and only append events and claims). Four resident blocks per
+// SM (64 registers): the redrawn layers' pass over a 100-day 1M-agent run took
 // 2.70 ms of kernel time against 2.89 ms with three (80 registers).
-// resident blocks per SM the per-source passes' registers must allow (three, 80
-// registers without spills, ran the 1M run 0.05 ms slower than four)
 #ifndef COVGPU_DYN_MIN_BLOCKS
 #define COVGPU_DYN_MIN_BLOCKS 4
 #endif
-template <bool LIK, bool WALK, int SPLIT>
-__global__ void __launch_bounds__(DYN_WARPS * 32, COVGPU_DYN_MIN_BLOCKS) k_dyn_pass(covgpu_state st, int t,
-                                                                                   int dyn_blocks) {
-  if (held(st, t)) return;
-  __shared__ union {
-    EdgeQueue e[DYN_WARPS];
-    SrcQueue s[SRC_WARPS];
+template <bool LIK, bool DYN, bool WALK>
+__global__ void __launch_bounds__(DYN_WARPS * 32, COVGPU_DYN_MIN_BLOCKS) k_source_pass(covgpu_state st, int t,
+                                                                                      int split) {
+  __shared__ union U {
+    EdgeQueue e[DYN ? DYN_WARPS : 1];
+    WalkShared w[WALK ? SRC_WARPS : 1];
+    __device__ U() {}
   } s_q;
-  if (!WALK || (int)blockIdx.x < dyn_blocks) dyn_body<LIK, SPLIT>(st, t, blockIdx.x, s_q.e);
-  else src_body<LIK, SPLIT>(st, t, (int64_t)blockIdx.x - dyn_blocks, s_q.s);
+  const bool both = DYN && WALK;
+  const int64_t vblock = both ? blockIdx.x >> 1 : blockIdx.x;
+  if (DYN && !(both && (blockIdx.x & 1))) dyn_body<LIK>(st, t, vblock, split, s_q.e);
+  else if (WALK) walk_body<LIK>(st, t, vblock, split, s_q.w);
+  pdl_trigger();
 }
 
-// The walk alone (a state without redrawn layers, or the stored layers' pass on
-// its own).
-template <bool LIK, int SPLIT>
-__global__ void __launch_bounds__(SRC_WARPS * 32) k_src_pass(covgpu_state st, int t) {
-  if (held(st, t)) return;
-  __shared__ SrcQueue s_q[SRC_WARPS];
-  src_body<LIK, SPLIT>(st, t, blockIdx.x, s_q);
+// dependent: launched as a dependent of the stream's previous kernel
+template <bool LIK>
+void launch_source_lik(const covgpu_state* st, int t, cudaStream_t s, bool dyn, bool walk, bool dependent) {
+  const int split = source_split(st);
+  const unsigned g = (unsigned)((split * st->n_agent_blocks + DYN_WARPS - 1) / DYN_WARPS);
+  const unsigned grid = dyn && walk ? 2 * g : g;
+  void (*k)(covgpu_state, int, int) = dyn && walk ? k_source_pass<LIK, true, true>
+                                                  : (dyn ? k_source_pass<LIK, true, false> : k_source_pass<LIK, false, true>);
+  if (dependent) launch_pdl(k, grid, DYN_WARPS * 32, 0, s, *st, t, split);
+  else k<<<grid, DYN_WARPS * 32, 0, s>>>(*st, t, split);
 }
-
-unsigned source_pass_blocks(const covgpu_state* st) {
-  return (unsigned)((source_split(st) * st->n_agent_blocks + DYN_WARPS - 1) / DYN_WARPS);
-}
-
-int launch_src_pass(const covgpu_state* st, int t, cudaStream_t s) {
-  if (st->n_tiles == 0 || st->src_walk == 0) return COVGPU_OK;
-  const unsigned grid = source_pass_blocks(st);
-  const bool one = source_split(st) == 1;
-  void (*k)(covgpu_state, int) = st->lik.factor ? (one ? k_src_pass<true, 1> : k_src_pass<true, 2>)
-                                                : (one ? k_src_pass<false, 1> : k_src_pass<false, 2>);
-  k<<<grid, SRC_WARPS * 32, 0, s>>>(*st, t);
-  return launch_status();
-}
-
-// the redrawn layers' pass; with_walk: also the walk of the stored layers (when
-// src_walk is on), in the same launch
-int launch_dyn_pass(const covgpu_state* st, int t, cudaStream_t s, bool with_walk) {
-  if (st->n_dynamic == 0) return COVGPU_OK;
-  const unsigned g = source_pass_blocks(st);
-  const bool walk = with_walk && st->n_tiles > 0 && st->src_walk != 0;
-  const unsigned grid = walk ? 2 * g : g;
-  void (*k)(covgpu_state, int, int);
-  if (source_split(st) == 1)
-    k = st->lik.factor ? (walk ? k_dyn_pass<true, true, 1> : k_dyn_pass<true, false, 1>)
-                       : (walk ? k_dyn_pass<false, true, 1> : k_dyn_pass<false, false, 1>);
-  else
-    k = st->lik.factor ? (walk ? k_dyn_pass<true, true, 2> : k_dyn_pass<true, false, 2>)
-                       : (walk ? k_dyn_pass<false, true, 2> : k_dyn_pass<false, false, 2>);
-  k<<<grid, DYN_WARPS * 32, 0, s>>>(*st, t, (int)g);
+int launch_source_pass(const covgpu_state* st, int t, cudaStream_t s, bool dyn, bool walk, bool dependent) {
+  dyn = dyn && st->n_dynamic > 0;
+  walk = walk && st->n_tiles > 0 && st->src_walk != 0;
+  if (!dyn && !walk) return COVGPU_OK;
+  if (st->lik.factor) launch_source_lik<true>(st, t, s, dyn, walk, dependent);
+  else launch_source_lik<false>(st, t, s, dyn, walk, dependent);
   return launch_status();
 }
 
@@ -1580,16 +1616,20 @@ int launch_stored_pass(const covgpu_state* st, int t, cudaStream_t s, bool with_
     launch_edge_tiles<false>(st, t, s);
   }
   const int rc = launch_status();
-  return (rc || !with_walk) ? rc : launch_src_pass(st, t, s);
+  return (rc || !with_walk) ? rc : launch_source_pass(st, t, s, false, true, false);
 }
+
+// every stored layer is walked on every day: the tile pass has nothing to do
+inline bool walk_all(const covgpu_state* st) { return st->src_walk == COVGPU_WALK_ALL; }
 
 // the stored layers' tiles, then the redrawn layers' sources (parts: 0 both, 1 or 2
 // one of them); the walk of the stored layers goes with the redrawn layers' pass
 // when both run, else with the stored layers'
 int launch_edge_pass(const covgpu_state* st, int t, cudaStream_t s, int parts = 0) {
+  if (walk_all(st)) return launch_source_pass(st, t, s, parts != 1, parts != 2, true);
   const bool walk_with_dyn = parts == 0 && st->n_dynamic > 0;
   const int rc = parts == 2 ? COVGPU_OK : launch_stored_pass(st, t, s, !walk_with_dyn);
-  return (rc || parts == 1) ? rc : launch_dyn_pass(st, t, s, walk_with_dyn);
+  return (rc || parts == 1) ? rc : launch_source_pass(st, t, s, true, walk_with_dyn, false);
 }
 
 // The same two passes side by side: they read the same start-of-day state and
@@ -1599,7 +1639,7 @@ int launch_edge_pass(const covgpu_state* st, int t, cudaStream_t s, int parts = 
 cudaStream_t g_side_stream = nullptr;
 cudaEvent_t g_fork_ev = nullptr, g_join_ev = nullptr;
 int launch_edge_pass_forked(const covgpu_state* st, int t, cudaStream_t s) {
-  if (st->n_tiles == 0 || st->n_dynamic == 0) return launch_edge_pass(st, t, s);
+  if (st->n_tiles == 0 || st->n_dynamic == 0 || walk_all(st)) return launch_edge_pass(st, t, s);
   if (!g_side_stream) {
     if (cudaStreamCreateWithFlags(&g_side_stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&g_fork_ev, cudaEventDisableTiming) != cudaSuccess ||
@@ -1608,7 +1648,7 @@ int launch_edge_pass_forked(const covgpu_state* st, int t, cudaStream_t s) {
   }
   if (cudaEventRecord(g_fork_ev, s) != cudaSuccess || cudaStreamWaitEvent(g_side_stream, g_fork_ev, 0) != cudaSuccess)
     return COVGPU_CUDA_ERROR;
-  int rc = launch_dyn_pass(st, t, g_side_stream, true);
+  int rc = launch_source_pass(st, t, g_side_stream, true, true, false);
   if (rc) return rc;
   if (cudaEventRecord(g_join_ev, g_side_stream) != cudaSuccess) return COVGPU_CUDA_ERROR;
   rc = launch_stored_pass(st, t, s, false);

@@ -200,6 +200,16 @@ __device__ __forceinline__ WarpBits warp_bits_scan(uint32_t word) {
   r.total = __shfl_sync(0xffffffffu, inc, 31);
   return r;
 }
+// position of the set bit of rank r (0 the lowest) of x, r < popc(x)
+__device__ __forceinline__ int nth_bit(uint32_t x, int r) {
+  int pos = 0;
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) {
+    const int c = __popc((x >> pos) & ((1u << s) - 1u));
+    if (r >= c) { r -= c; pos += s; }
+  }
+  return pos;
+}
 __device__ __forceinline__ int warp_bits_nth(const WarpBits& wb, int nw, int idx, int& bit) {
   int src = 0;
   for (int k = 1; k < nw; ++k)
@@ -207,7 +217,7 @@ __device__ __forceinline__ int warp_bits_nth(const WarpBits& wb, int nw, int idx
   const uint32_t wd = __shfl_sync(0xffffffffu, wb.word, src);
   const int pk = __shfl_sync(0xffffffffu, wb.pre, src);
   const int r = idx - pk;
-  bit = (r >= 0 && r < __popc(wd)) ? (int)__fns(wd, 0u, r + 1) : 0;
+  bit = (r >= 0 && r < __popc(wd)) ? nth_bit(wd, r) : 0;
   return src;
 }
 

@@ -300,8 +300,11 @@ __device__ __forceinline__ bool frac_less(uint64_t lhs, int nbits, float p) {
   const uint64_t rem = mant & ((1ull << (-sh)) - 1ull);
   return lhs < q || (lhs == q && rem != 0);
 }
-// Philox words -> the (0,1) doubles of u01_52 / u01_32, compared with p exactly
+// Philox words -> the (0,1) doubles of u01_52 / u01_32, compared with p exactly.
+// Most draws are far above a small p: the uniform is at least its top 24 bits
+// (exact in float32, as is p * 2^24), which settles those in three instructions.
 __device__ __forceinline__ bool bern52(uint32_t a, uint32_t b, float p) {
+  if ((float)(a >> 8) >= __fmul_rn(p, 16777216.0f)) return false;
   const uint64_t k = ((uint64_t)(a >> 6) << 26) | (uint64_t)(b >> 6);
   return frac_less(2 * k + 1, 53, p);
 }

@@ -117,7 +117,7 @@ __device__ __noinline__ void mark_contacts(const covgpu_state& st, const covgpu_
           atomicOr(contact + (g >> 5), 1u << (g & 31));
         }
         for (uint32_t k = b2 + sub; k < e2; k += MARK_LANES) {
-          const int32_t g = L.p1[L.perm2[k]];
+          const int32_t g = L.rev1 ? L.rev1[k] : L.p1[L.perm2[k]];
           atomicOr(contact + (g >> 5), 1u << (g & 31));
         }
       }
@@ -600,13 +600,14 @@ __global__ void k_rev_offsets(const int64_t* offsets, int64_t n, uint32_t* rp2) 
   if (a <= n) rp2[a] = (uint32_t)offsets[a];
 }
 __global__ void k_rev_place(const int32_t* p2, int64_t n_edges, int64_t off, int64_t n_local, int64_t* cursor,
-                            uint32_t* perm2) {
+                            uint32_t* perm2, const int32_t* p1, int32_t* rev1) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n_edges) return;
   const int64_t a = (int64_t)p2[e] - off;
   if (a < 0 || a >= n_local) return;
   const unsigned long long pos = atomicAdd(reinterpret_cast<unsigned long long*>(cursor + a), 1ull);
   perm2[pos] = (uint32_t)e;
+  if (rev1) rev1[pos] = p1[e];
 }
 
 }  // namespace
@@ -662,8 +663,8 @@ int64_t covgpu_trace_index_scratch(int64_t n_local) {
   return 2 * (n_local + 1) + (int64_t)scan_blocks_for(n_local, SCAN_TILE) + 1;
 }
 
-int covgpu_trace_index(const int32_t* p1, const int32_t* p2, int64_t n_edges, int64_t agent_off, int64_t n_local,
-                       uint32_t* rp1, uint32_t* rp2, uint32_t* perm2, int64_t* scratch, void* stream) {
+int covgpu_agent_index(const int32_t* p1, const int32_t* p2, int64_t n_edges, int64_t agent_off, int64_t n_local,
+                       uint32_t* rp1, uint32_t* rp2, uint32_t* perm2, int32_t* rev1, int64_t* scratch, void* stream) {
   if (n_edges < 1 || n_edges > 0xFFFFFFFFLL || n_local < 1 || agent_off < 0 || !p1 || !p2 || !rp1 || !rp2 ||
       !perm2 || !scratch)
     return COVGPU_BADARG;
@@ -677,8 +678,13 @@ int covgpu_trace_index(const int32_t* p1, const int32_t* p2, int64_t n_edges, in
   int rc = scan_i64(counts, offsets, n_local, tiles, s);
   if (rc) return rc;
   k_rev_offsets<<<grid_for(n_local + 1, 256, 1 << 30), 256, 0, s>>>(offsets, n_local, rp2);
-  k_rev_place<<<grid_for(n_edges, 256, 1 << 30), 256, 0, s>>>(p2, n_edges, agent_off, n_local, offsets, perm2);
+  k_rev_place<<<grid_for(n_edges, 256, 1 << 30), 256, 0, s>>>(p2, n_edges, agent_off, n_local, offsets, perm2, p1, rev1);
   return launch_status();
+}
+
+int covgpu_trace_index(const int32_t* p1, const int32_t* p2, int64_t n_edges, int64_t agent_off, int64_t n_local,
+                       uint32_t* rp1, uint32_t* rp2, uint32_t* perm2, int64_t* scratch, void* stream) {
+  return covgpu_agent_index(p1, p2, n_edges, agent_off, n_local, rp1, rp2, perm2, nullptr, scratch, stream);
 }
 
 }  // extern "C"

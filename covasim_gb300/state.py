@@ -261,18 +261,25 @@ def ili_agents(seed, t, n, n_ili):
     return np.sort(rng.choice(int(n), int(n_ili), replace=False)).astype(np.int32)
 
 
-# Default of covgpu_state.src_walk for a state with a redrawn layer: the stored
-# layers are walked from the day's sources while fewer than 1/128 of a sim's agents
-# are infectious, and streamed otherwise (results are the same either way). The
-# walk then runs in the redrawn layers' launch, beside their draws: on the 1M-agent
-# hybrid run, 18.45 -> 18.0 ms per run (thresholds 1/64 to 1/512 within 0.1 ms of
-# each other). Without a redrawn layer the walk is a launch of its own after the
-# tile pass, which costs about 12 us a day before any source is walked, and the
-# stored layers are streamed (0), unless the state holds at least SRC_WALK_MIN_EDGES
-# stored edges: then the day's stream is long enough for the walk to pay even as a
-# launch of its own (256 random-population sims, 320M edges, 120 days: 262 -> 238 ms
-# per batched run walking below 1/64 infectious).
+# When the stored layers are walked from the day's sources (covgpu_state.src_walk;
+# results are the same either way). BatchState.src_walk is the threshold k of a
+# state with a redrawn layer (SRC_WALK) or of one whose stored edges make a day's
+# stream long (SRC_WALK_BIG, from SRC_WALK_MIN_EDGES edges); both build the agent
+# index the walk needs, as tracing does. Until set_src_walk asks for a threshold,
+# _walk_mode refines it from sizes once every stored layer has its index:
+# * no redrawn layer: walked every day, and the tile pass is not launched (96
+#   random-population sims, 115M edges, 120 days: 83.5 ms a batched run, 106.3 ms
+#   walking below 1/64 infectious and 107.2 ms below 1/8, two launches a day);
+# * a redrawn layer, below SRC_WALK_ALL_AGENTS agents: walked every day, one launch
+#   with the redrawn layer's pass instead of a fork and join of two (300,000 agents,
+#   testing: 6.97 ms a run, 7.29 below 1/128); above, the stream beside the redrawn
+#   layer's pass is faster on the busy days (1M agents: 15.9 ms below 1/16, 17.3
+#   every day, 16.0 below 1/128; 10M: 105.4, 105.2, 111.3);
+# * with the likelihood, whose walk takes the layers one after another, SRC_WALK
+#   (100,000 agents: 7.96 ms, 8.44 every day).
 SRC_WALK = 128
+SRC_WALK_REDRAWN = 16
+SRC_WALK_ALL_AGENTS = 500_000
 SRC_WALK_BIG = 64
 SRC_WALK_MIN_EDGES = 50_000_000
 
@@ -305,6 +312,7 @@ class BatchState:
         else:
             stored = sum(len(ly['p1']) for sp in specs for ly in sp.layers)
             self.src_walk = SRC_WALK_BIG if stored >= SRC_WALK_MIN_EDGES else 0
+        self._walk_default = True  # until set_src_walk
         self._index_pending = []  # stored segments whose agent index is built on demand
         self._index_tensors = []
         if not torch.cuda.is_available():
@@ -706,15 +714,14 @@ class BatchState:
 
     def _build_index(self, rec, sp, off, n_edges):
         dev, n = self.device, sp.n
-        rp1 = torch.empty(n + 1, dtype=I32, device=dev)
-        rp2 = torch.empty(n + 1, dtype=I32, device=dev)
-        perm2 = torch.empty(n_edges, dtype=I32, device=dev)
+        rp = torch.empty((2, n + 1), dtype=I32, device=dev)
+        rev = torch.empty((2, n_edges), dtype=I32, device=dev)  # perm2 and rev1
         scratch = torch.empty(int(self.lib.covgpu_trace_index_scratch(n)), dtype=I64, device=dev)
-        L.call('covgpu_trace_index', rec.p1, rec.p2, int(n_edges), int(off), int(n), rp1.data_ptr(), rp2.data_ptr(),
-               perm2.data_ptr(), scratch.data_ptr(), _stream())
-        rec.rp1, rec.rp2, rec.perm2 = rp1.data_ptr(), rp2.data_ptr(), perm2.data_ptr()
+        L.call('covgpu_agent_index', rec.p1, rec.p2, int(n_edges), int(off), int(n), *(x.data_ptr() for x in (*rp, *rev)),
+               scratch.data_ptr(), _stream())
+        rec.rp1, rec.rp2, rec.perm2, rec.rev1 = (x.data_ptr() for x in (*rp, *rev))
         self._index_scratch = scratch  # kept until the build has run on the stream
-        return [rp1, rp2, perm2]
+        return [rp, rev]
 
     def _tile_segments(self):
         """Each segment's first tile and the tile count for the current edge tile size
@@ -755,12 +762,25 @@ class BatchState:
     def resident_possible(self):
         return int(self.lib.covgpu_edge_resident_bytes(self.cstate_ptr)) > 0
 
+    def _walk_mode(self):
+        """covgpu_state.src_walk: the threshold asked for (-1: every day), or the
+        default rule (above) until one is asked for."""
+        k = int(self.src_walk)
+        indexed = all(rec.dynamic or rec.rp1 for rec in self.segments)
+        if self._walk_default and indexed:
+            if not any(rec.dynamic for rec in self.segments):
+                k = -1
+            elif not self.lik_active:
+                k = -1 if self.n < SRC_WALK_ALL_AGENTS else SRC_WALK_REDRAWN
+        return L.WALK_ALL if indexed and k == -1 else k
+
     def set_src_walk(self, k):
         """Quiet-day walk of the stored layers (covgpu_state.src_walk): k > 0 walks
         a layer from the day's sources while its sim's infectious agents x k are
         fewer than its agents, 0 never, -1 always (building the layers' agent index
         first). Results do not depend on it."""
         self.src_walk = int(k)
+        self._walk_default = False
         if self.src_walk and self._index_pending:
             for rec, sp, off, n_edges in self._index_pending:
                 self._index_tensors += self._build_index(rec, sp, off, n_edges)
@@ -901,7 +921,7 @@ class BatchState:
         st.n_segments = len(self.segments)
         st.n_tiles = self.n_tiles
         st.n_dynamic = self.n_dynamic
-        st.src_walk = int(self.src_walk)
+        st.src_walk = self._walk_mode()
         st.n_agent_blocks = self.n_agent_blocks
         st.edge_tile = self.edge_tile
         st.edge_resident = int(self.edge_resident)

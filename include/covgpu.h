@@ -224,6 +224,7 @@ typedef struct covgpu_sim_params {
  * distribution: dyn_cdf[k] = floor(2^64 * P(count <= k)) for k < dyn_k - 1
  * and dyn_cdf[dyn_k - 1] = 2^64 - 1, with dyn_k <= COVGPU_DYN_MAX_LIST. */
 #define COVGPU_DYN_MAX_LIST 1024
+#define COVGPU_WALK_ALL (-2)      /* covgpu_state.src_walk */
 typedef struct covgpu_layer {
   const int32_t* p1;              /* global agent indices, sorted ascending (static) */
   const int32_t* p2;
@@ -239,9 +240,10 @@ typedef struct covgpu_layer {
   int32_t dyn_k;                  /* dynamic: entries of dyn_cdf                    */
   /* agent index of a stored layer (NULL: none; covgpu_trace_index): the agent
    * a's edges as p1 are [rp1[a], rp1[a+1]), as p2 the edges perm2[rp2[a] ..
-   * rp2[a+1]) (a local to the sim). With it the edge pass walks the layer from
-   * the day's sources on days its sim has few infectious agents, and the
-   * tracing pass visits only the traced agents' edges. */
+   * rp2[a+1]) (a local to the sim), and rev1[k] = p1[perm2[k]] (or NULL: read
+   * through perm2). With it the edge pass can walk the layer from the day's
+   * sources (covgpu_state.src_walk), and the tracing pass visits only the traced
+   * agents' edges. */
   const uint32_t* rp1;
   const uint32_t* rp2;
   const uint32_t* perm2;
@@ -251,6 +253,7 @@ typedef struct covgpu_layer {
                                      rel_sus, times quar_factor when above 1); the
                                      edge pass thins each source's entries by it     */
   int32_t _pad2;
+  const int32_t* rev1;
 } covgpu_layer;
 
 /* One agent block of the agent kernel: agents [begin, end) of one sim. */
@@ -362,11 +365,12 @@ typedef struct covgpu_state {
   uint32_t* trace_bits;           /* [ceil(n/32)] agents traced today                */
   uint32_t* contact_bits;         /* [n_contact_layers][ceil(n/32)] contacts found   */
   int32_t n_contact_layers;       /* max layers over sims                            */
-  int32_t src_walk;               /* indexed stored layers on quiet days: k > 0 walks a
-                                     layer from the day's sources while its sim's
-                                     infectious agents x k < its agents; 0 never,
-                                     -1 always (the streamed and walked passes give
-                                     the same results)                             */
+  int32_t src_walk;               /* indexed stored layers: k > 0 walks a layer from the
+                                     day's sources while its sim's infectious agents x
+                                     k < its agents; 0 never, -1 always, COVGPU_WALK_ALL
+                                     always and every stored layer has its index (the
+                                     tile pass is not launched). The streamed and the
+                                     walked pass give the same results               */
   int32_t* pending_quar;          /* [R][n] end day of a quarantine starting on day
                                      s (slot s mod R), -1: none                      */
   uint32_t* trace_count;          /* [n_sims] agents traced today                    */
@@ -571,6 +575,9 @@ int covgpu_lik_targets(const covgpu_state* st, int32_t t, void* stream);
 int64_t covgpu_trace_index_scratch(int64_t n_local);
 int covgpu_trace_index(const int32_t* p1, const int32_t* p2, int64_t n_edges, int64_t agent_off, int64_t n_local,
                        uint32_t* rp1, uint32_t* rp2, uint32_t* perm2, int64_t* scratch, void* stream);
+/* The same with rev1 [n_edges], the p1 of each entry of perm2 (NULL: without). */
+int covgpu_agent_index(const int32_t* p1, const int32_t* p2, int64_t n_edges, int64_t agent_off, int64_t n_local,
+                       uint32_t* rp1, uint32_t* rp2, uint32_t* perm2, int32_t* rev1, int64_t* scratch, void* stream);
 
 /* infect() for the winning event of each target. */
 int covgpu_infect_claims(const covgpu_state* st, int32_t t, void* stream);
