@@ -36,19 +36,13 @@ using namespace covgpu;
 
 namespace {
 
-// resident blocks per SM that the register budget of the agent pass must allow
-// (0: the compiler's choice); the pass's grid is one wave of them. Three blocks
-// ran a whole 1M-agent run (one CUDA graph) 0.8 ms faster than four and 2.3 ms
-// faster than five (both spilling); bounding the infect pass the same way
-// changed nothing.
-#ifndef COVGPU_AGENT_MIN_BLOCKS
-#define COVGPU_AGENT_MIN_BLOCKS 3
-#endif
-#if COVGPU_AGENT_MIN_BLOCKS
-#define AGENT_BOUNDS __launch_bounds__(AGENT_THREADS, COVGPU_AGENT_MIN_BLOCKS)
-#else
-#define AGENT_BOUNDS __launch_bounds__(AGENT_THREADS)
-#endif
+// resident blocks per SM that the register budget of the agent pass must allow; the
+// pass's grid is one wave of them. In place, three blocks ran a whole 1M-agent run
+// 0.8 ms faster than four and 2.3 ms faster than five (both spilling); with the
+// efficacy queue, four (64 registers) ran a 10M-agent one 0.7 ms faster than three
+// and 6.4 ms faster than five.
+constexpr int AGENT_BLOCKS = 3;
+constexpr int AGENT_QUEUE_BLOCKS = 4;
 constexpr int EQ_ROUND = 32 * EDGE_VEC;  // most candidates one warp appends per round (one per edge)
 constexpr int EQ_CAP = 32 + EQ_ROUND;  // candidate queue entries per warp: fewer than 32 left over + one round
 static_assert(2 * EDGE_TILE_MAX <= 65536, "queue entries pack (edge within the tile, direction) in 16 bits");
@@ -112,6 +106,52 @@ constexpr uint64_t FLOW_SLOTS =
 static_assert(COVGPU_N_RES_INT <= 64, "six-bit slots");
 static_assert(DW_VAR + COVGPU_MAX_VARIANTS <= DW_SRC, "day-word layout");
 
+// check_immunity (immunity.py:303-350) of agent i: the daily efficacies against every variant (float-float, one
+// rounding), a target's records (rs: its rel_sus with sign bit = quarantined, 0: not
+// a target) and the sums of levels. meta: recovered variant | recovered << 8 | the
+// vaccinated flag.
+__device__ __forceinline__ void ve_agent(const covgpu_state& st, const covgpu_sim_params& sp, int64_t i, float nab,
+                                         uint32_t rs, uint32_t meta, int full_imm, const float (*s_ln_tab)[2],
+                                         const float* s_ln_inv, const float (*s_exp_tab)[2], long long& sus_fx,
+                                         long long& symp_fx) {
+  ff ln_nab = ff{0.0f, 0.0f};
+  bool have_ln = false;
+  for (int v = 0; v < sp.n_variants; ++v) {
+    ff ln_imm;  // imm = max(natural, vaccine); ln(imm) from the host's tables
+    const float imm = imm_of(st, sp, i, v, meta, (meta >> 8) & 1u, meta & 0xFFu, ln_imm);
+    float a = 0.0f, b = 0.0f, c = 0.0f;
+    if (nab > 0.0f && imm > 0.0f) {  // eff = nab * imm > 0; else every efficacy is 0
+      if (!have_ln) { ln_nab = ff_log(nab, s_ln_tab, s_ln_inv); have_ln = true; }
+      const ff ln_eff = ff_add(ln_nab, ln_imm);
+      a = ve_axis(sp, 0, ln_eff, s_exp_tab);
+      b = ve_axis(sp, 1, ln_eff, s_exp_tab);
+      if (full_imm) c = ve_axis(sp, 2, ln_eff, s_exp_tab);
+    }
+    const int64_t off = (int64_t)v * st.n + i;
+    st.sus_imm[off] = a;
+    st.symp_imm[off] = b;
+    if (full_imm) st.sev_imm[off] = c;
+    if (rs & 0x7FFFFFFFu)
+      st.tgt_rec[off] = __uint_as_float(__float_as_uint(__fmul_rn(__uint_as_float(rs & 0x7FFFFFFFu),
+                                                                  __fsub_rn(1.0f, a))) | (rs & 0x80000000u));
+    if (a != 0.0f || b != 0.0f) {
+      sus_fx += __float2ll_rn(__fmul_rn(a, 4294967296.0f));
+      symp_fx += __float2ll_rn(__fmul_rn(b, 4294967296.0f));
+    }
+  }
+}
+
+// The agents of one warp with NAbs and an immunity to scale (about 350 instructions
+// a variant), queued across the agent blocks it walks and drained 32 at a time on full warps;
+// in place, the whole warp runs them for the few of its 32 agents that have
+// recovered (k_agent_step<QUEUE>, agent_queue).
+constexpr int VEQ_CAP = 64;  // fewer than 32 left over + one agent block's 32
+struct VeQueue {
+  uint32_t i[VEQ_CAP];
+  float nab[VEQ_CAP];
+  uint32_t rs[VEQ_CAP], meta[VEQ_CAP];
+};
+
 // One agent block (up to 256 agents of one sim, thread k on agent begin + k):
 // closes day t-1 and runs day t's checks for its agents. Counts go to per-lane
 // accumulators: the agents' flag words (for the stocks) and day words (for the
@@ -122,9 +162,10 @@ static_assert(DW_VAR + COVGPU_MAX_VARIANTS <= DW_SRC, "day-word layout");
 // reductions, independent of order, and no float64 work per agent). full_imm: also store sev_imm (read only by infect(), which
 // recomputes it for the agents it infects; stored on the last day of a launch
 // sequence, so that the state a caller reads afterwards holds the reference's array).
+template <bool QUEUE>
 __device__ __forceinline__ void agent_block_step(const covgpu_state& st, const covgpu_agent_block& blk,
                                                  const AgentIn& in, int t, int do_prev, int do_day, int full_imm,
-                                                 int steady,
+                                                 int steady, VeQueue& vq, int& qn,
                                                  const float (*s_ln_tab)[2], const float* s_ln_inv,
                                                  const float (*s_exp_tab)[2],
                                                  long long& nab_fx, long long& sus_fx, long long& symp_fx,
@@ -179,7 +220,8 @@ __device__ __forceinline__ void agent_block_step(const covgpu_state& st, const c
   }
 
   // ---------------------------------------------------------- day t
-  uint32_t src_bit = 0, tgt_bit = 0;
+  uint32_t src_bit = 0, tgt_bit = 0, ve_meta = 0, ve_rs = 0;
+  bool ve = false;  // to the queue
   if (do_day) {
     unsigned c_inf = 0, c_symp = 0, c_sev = 0, c_crit = 0, c_rec = 0, c_dead = 0, c_kdead = 0;
     int inf_v = -1;
@@ -262,30 +304,23 @@ __device__ __forceinline__ void agent_block_step(const covgpu_state& st, const c
         // for it, symp_imm_of), and the target record is rel_sus itself
         if (is_tgt)
           for (int v = 0; v < nv; ++v) st.tgt_rec[(int64_t)v * st.n + i] = __uint_as_float(__float_as_uint(rs) | tq);
-      } else if (waning) {  // check_immunity, immunity.py:303-350 (float-float, one rounding)
+      } else if (waning) {
         const bool was_inf = tf >= a_dr;  // false for NaN
-        const float nab = nab_now;
-        ff ln_nab = ff{0.0f, 0.0f};
-        bool have_ln = false;
-        for (int v = 0; v < nv; ++v) {
-          ff ln_imm;  // imm = max(natural, vaccine); ln(imm) from the host's tables
-          const float imm = imm_of(st, sp, i, v, f, was_inf, rv, ln_imm);
-          float a = 0.0f, b = 0.0f, c = 0.0f;
-          if (nab > 0.0f && imm > 0.0f) {  // eff = nab * imm > 0; else every efficacy is 0
-            if (!have_ln) { ln_nab = ff_log(nab, s_ln_tab, s_ln_inv); have_ln = true; }
-            const ff ln_eff = ff_add(ln_nab, ln_imm);
-            a = ve_axis(sp, 0, ln_eff, s_exp_tab);
-            b = ve_axis(sp, 1, ln_eff, s_exp_tab);
-            if (full_imm) c = ve_axis(sp, 2, ln_eff, s_exp_tab);
-          }
-          const int64_t off = (int64_t)v * st.n + i;
-          st.sus_imm[off] = a;
-          st.symp_imm[off] = b;
-          if (full_imm) st.sev_imm[off] = c;
-          if (is_tgt) st.tgt_rec[off] = __uint_as_float(__float_as_uint(__fmul_rn(rs, __fsub_rn(1.0f, a))) | tq);
-          if (a != 0.0f || b != 0.0f) {
-            sus_fx += __float2ll_rn(__fmul_rn(a, 4294967296.0f));
-            symp_fx += __float2ll_rn(__fmul_rn(b, 4294967296.0f));
+        const uint32_t rsq = is_tgt ? __float_as_uint(rs) | tq : 0u;
+        const uint32_t meta = (f & B_VACC) | (was_inf ? 0x100u : 0u) | rv;
+        if (!QUEUE) {
+          ve_agent(st, sp, i, nab_now, rsq, meta, full_imm, s_ln_tab, s_ln_inv, s_exp_tab, sus_fx, symp_fx);
+        } else if (nab_now > 0.0f && (was_inf || (f & B_VACC))) {
+          ve = true;
+          ve_rs = rsq;
+          ve_meta = meta;
+        } else {  // no NAbs, or immune to nothing: every efficacy is 0
+          for (int v = 0; v < nv; ++v) {
+            const int64_t off = (int64_t)v * st.n + i;
+            st.sus_imm[off] = 0.0f;
+            st.symp_imm[off] = 0.0f;
+            if (full_imm) st.sev_imm[off] = 0.0f;
+            if (is_tgt) st.tgt_rec[off] = __uint_as_float(rsq);
           }
         }
       }
@@ -318,6 +353,17 @@ __device__ __forceinline__ void agent_block_step(const covgpu_state& st, const c
     // new infectious by variant and the roles, one bit each of the day word;
     // transposed, lanes 30 and 31 hold the role bitmaps' words of this warp's 32
     // agents (the 32-aligned word (i - lane) / 32)
+    if (QUEUE) {
+      const unsigned vem = __ballot_sync(0xffffffffu, ve);
+      if (ve) {
+        const int k = qn + __popc(vem & ((1u << lane) - 1u));
+        vq.i[k] = (uint32_t)i;
+        vq.nab[k] = nab_now;
+        vq.rs[k] = ve_rs;
+        vq.meta[k] = ve_meta;
+      }
+      qn += __popc(vem);
+    }
     const uint32_t dw = valid ? (c_inf | c_symp << 1 | c_sev << 2 | c_crit << 3 | c_rec << 4 | c_dead << 5 |
                                  c_kdead << 6 | ((f & B_SEV) ? 1u << 7 : 0u) | ((f & B_CRIT) ? 1u << 8 : 0u) |
                                  (inf_v >= 0 ? 1u << (DW_VAR + inf_v) : 0u) | src_bit << DW_SRC |
@@ -412,7 +458,8 @@ __device__ __noinline__ void agent_flush(const covgpu_state& st, int sim, int t,
 // flight while the current one is processed, no barrier separates agent blocks of
 // one sim, and the counters go to the results once per sim a block touched
 // instead of once per 256 agents.
-__global__ void AGENT_BOUNDS k_agent_step(covgpu_state st, int t, int do_prev, int do_day, int full_imm, int steady) {
+template <bool QUEUE>
+__global__ void __launch_bounds__(AGENT_THREADS, QUEUE ? AGENT_QUEUE_BLOCKS : AGENT_BLOCKS) k_agent_step(covgpu_state st, int t, int do_prev, int do_day, int full_imm, int steady) {
   const int64_t nb = st.n_agent_blocks;
   const int64_t per = (nb + gridDim.x - 1) / gridDim.x;
   int64_t b = (int64_t)blockIdx.x * per;
@@ -424,6 +471,9 @@ __global__ void AGENT_BOUNDS k_agent_step(covgpu_state st, int t, int do_prev, i
   __shared__ float s_ln_tab[COVGPU_LN_N][2];
   __shared__ float s_ln_inv[COVGPU_LN_N];
   __shared__ float s_exp_tab[COVGPU_EXP_N][2];
+  __shared__ VeQueue s_vq[QUEUE ? AGENT_THREADS / 32 : 1];
+  VeQueue& vq = s_vq[QUEUE ? threadIdx.x >> 5 : 0];
+  int qn = 0;
   for (int k = threadIdx.x; k < 2 * COVGPU_LN_N; k += blockDim.x) (&s_ln_tab[0][0])[k] = (&COVGPU_LN_TAB[0][0])[k];
   for (int k = threadIdx.x; k < COVGPU_LN_N; k += blockDim.x) s_ln_inv[k] = COVGPU_LN_INV[k];
   for (int k = threadIdx.x; k < 2 * COVGPU_EXP_N; k += blockDim.x) (&s_exp_tab[0][0])[k] = (&COVGPU_EXP_TAB[0][0])[k];
@@ -454,8 +504,20 @@ __global__ void AGENT_BOUNDS k_agent_step(covgpu_state st, int t, int do_prev, i
       const int64_t ni = nblk.begin + threadIdx.x;
       nxt = agent_load(st, ni, ni < nblk.end, st.sims[nblk.sim].use_waning != 0);
     }
-    agent_block_step(st, blk, cur, t, do_prev, do_day, full_imm, steady, s_ln_tab, s_ln_inv, s_exp_tab, nab_fx, sus_fx,
-                     symp_fx, acc_prev, acc_day);
+    agent_block_step<QUEUE>(st, blk, cur, t, do_prev, do_day, full_imm, steady, vq, qn, s_ln_tab, s_ln_inv, s_exp_tab,
+                            nab_fx, sus_fx, symp_fx, acc_prev, acc_day);
+    if (QUEUE) {
+      const bool last = !more || nblk.sim != sim;  // of this sim: the queue is emptied
+      __syncwarp();
+      while (qn >= 32 || (last && qn > 0)) {
+        const int base = qn >= 32 ? qn - 32 : 0, k = base + (threadIdx.x & 31);
+        if (k < qn)
+          ve_agent(st, st.sims[sim], vq.i[k], vq.nab[k], vq.rs[k], vq.meta[k], full_imm, s_ln_tab, s_ln_inv, s_exp_tab,
+                   sus_fx, symp_fx);
+        qn = base;
+      }
+      __syncwarp();
+    }
     if (!more) break;
     ++b;
     if (nblk.sim != sim) {
@@ -2290,28 +2352,29 @@ GraphEntry g_graphs[N_GRAPHS];
 int g_graph_next = 0;
 cudaStream_t g_capture_stream = nullptr;  // private stream for captures (the legacy stream cannot capture)
 
-// Grid of the agent pass: one wave of resident blocks (the SM count of the current
-// device times the blocks per SM the pass's registers allow), or fewer when the
-// state has fewer agent blocks. Any grid gives the same results.
-unsigned agent_grid(const covgpu_state* st) {
-  static const int64_t wave = [] {
-    int dev = 0, sms = 0, per_sm = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_agent_step, AGENT_THREADS, 0) != cudaSuccess) {
-      cudaGetLastError();
-      return (int64_t)1 << 30;  // no wave bound: one block per agent block
-    }
-    return (int64_t)(sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
-  }();
-  const int64_t nb = st->n_agent_blocks;
-  return (unsigned)(nb < wave ? (nb > 0 ? nb : 1) : wave);
+// The agent pass: one wave of resident blocks, or fewer when the state has fewer
+// agent blocks (any grid, and either form, gives the same results). The efficacy
+// queue pays where a warp walks enough agent blocks to fill it: a run took 23.7 ms
+// with it and 24.2 in place with 2M agents (13 agent blocks a resident block), 35.7
+// and 37.0 with 5M, 93.2 and 106.1 with 10M (three variants), 81.0 and 85.0 with 96
+// sims of 11.4M; 19.1 and 19.0 with 1.5M, 16.4 and 16.1 with 1M (6).
+constexpr int64_t AGENT_QUEUE_MIN = 12;  // agent blocks per resident block
+struct AgentLaunch {
+  void (*kernel)(covgpu_state, int, int, int, int, int);
+  unsigned grid;
+};
+AgentLaunch agent_launch(const covgpu_state* st) {
+  static const int64_t wave = wave_blocks(k_agent_step<false>, AGENT_THREADS);
+  static const int64_t queue_wave = wave_blocks(k_agent_step<true>, AGENT_THREADS);
+  if (st->n_agent_blocks >= AGENT_QUEUE_MIN * queue_wave) return {k_agent_step<true>, wave_grid(st, queue_wave)};
+  return {k_agent_step<false>, wave_grid(st, wave)};
 }
 
 int enqueue_days(const covgpu_state* st, int t0, int t1, int open_prev, int close_last, cudaStream_t s) {
+  const AgentLaunch agent = agent_launch(st);
   for (int t = t0; t < t1; ++t) {
     if (st->hold) k_rescale_check<<<1, 128, 0, s>>>(*st, t);
-    launch_pdl(k_agent_step, agent_grid(st), AGENT_THREADS, 0, s, *st, t, (t > t0 || open_prev) ? 1 : 0, 1,
+    launch_pdl(agent.kernel, agent.grid, AGENT_THREADS, 0, s, *st, t, (t > t0 || open_prev) ? 1 : 0, 1,
                t == t1 - 1 ? 1 : 0, t > t0 ? 1 : 0);
     if (t < st->import_days) k_import_day<<<IMPORT_BLOCKS, 256, 0, s>>>(*st, t);
     launch_test_trace(st, t, s);
@@ -2320,7 +2383,7 @@ int enqueue_days(const covgpu_state* st, int t0, int t1, int open_prev, int clos
     launch_lik_targets(st, t, s);
     launch_pdl(k_infect_claims, (unsigned)grid_for(st->n / 8 + 1, 256, 152 * 4), 256, 0, s, *st, t);
   }
-  if (close_last) launch_pdl(k_agent_step, agent_grid(st), AGENT_THREADS, 0, s, *st, t1, 1, 0, 0, 1);
+  if (close_last) launch_pdl(agent.kernel, agent.grid, AGENT_THREADS, 0, s, *st, t1, 1, 0, 0, 1);
   return launch_status();
 }
 
@@ -2385,7 +2448,8 @@ int covgpu_agent_step(const covgpu_state* st, int32_t t, int32_t do_prev, int32_
   if (t < 0 || t >= 0xFFFF) return COVGPU_BADARG;
   if (do_day & ~(1 | COVGPU_DAY_STEADY)) return COVGPU_BADARG;
   const int day = do_day & 1, steady = (!day || (do_day & COVGPU_DAY_STEADY)) ? 1 : 0;
-  k_agent_step<<<agent_grid(st), AGENT_THREADS, 0, S(stream)>>>(*st, t, do_prev, day, 1, steady);
+  const AgentLaunch agent = agent_launch(st);
+  agent.kernel<<<agent.grid, AGENT_THREADS, 0, S(stream)>>>(*st, t, do_prev, day, 1, steady);
   return launch_status();
 }
 
