@@ -154,6 +154,13 @@ class State(C.Structure):
     ]
 
 
+class Span(C.Structure):
+    _fields_ = [('dst', C.c_void_p), ('src', C.c_void_p), ('bytes', C.c_int64), ('fill', C.c_int32),
+                ('_pad', C.c_int32)]
+
+
+OUTCOME_BLOCKS = 304  # COVGPU_OUTCOME_BLOCKS
+
 _lib = None
 
 
@@ -194,6 +201,12 @@ def lib():
         L.covgpu_check_immunity.argtypes = [sp, i32, i32, C.c_uint32, vp]
         L.covgpu_update_nab.argtypes = [sp, i32, i32, vp, i64, vp]
         L.covgpu_update_peak_nab.argtypes = [sp, i32, i32, vp, i64, vp, DurPar, f32, C.c_double, i32, vp]
+        L.covgpu_infect_sims.argtypes = [sp, i32, vp, vp, i64, i32, i32, i32, vp]
+        L.covgpu_infect_sims.restype = C.c_int
+        L.covgpu_copy_spans.argtypes = [C.POINTER(Span), i32, vp]
+        L.covgpu_copy_spans.restype = C.c_int
+        L.covgpu_outcome_sums.argtypes = [vp, vp, vp, i64, vp, vp]
+        L.covgpu_outcome_sums.restype = C.c_int
         L.covgpu_import_day.argtypes = [sp, i32, vp]
         L.covgpu_rescale_check.argtypes = [sp, i32, vp]
         L.covgpu_layer_lists.argtypes = [sp, i32, i32, i64, i64, vp, vp, vp, vp]
@@ -258,7 +271,7 @@ POP_FUNCS = ['covgpu_pop_ages', 'covgpu_pop_members', 'covgpu_pop_random_counts'
 EXPORTED = ['covgpu_version', 'covgpu_abi_layout', 'covgpu_viral_load', 'covgpu_trans_sus', 'covgpu_infections_scratch_bytes',
             'covgpu_infections', 'covgpu_infections_find', 'covgpu_infections_emit',
             'covgpu_infections_noalloc', 'covgpu_agent_step', 'covgpu_edge_pass', 'covgpu_infect_claims',
-            'covgpu_infect_list', 'covgpu_import_day', 'covgpu_rescale_check', 'covgpu_layer_lists', 'covgpu_run_days', 'covgpu_test_trace',
+            'covgpu_infect_list', 'covgpu_infect_sims', 'covgpu_copy_spans', 'covgpu_outcome_sums', 'covgpu_import_day', 'covgpu_rescale_check', 'covgpu_layer_lists', 'covgpu_run_days', 'covgpu_test_trace',
             'covgpu_lik_targets', 'covgpu_trace_index_scratch', 'covgpu_trace_index', 'covgpu_agent_index', 'covgpu_edge_resident_bytes',
             'covgpu_check', 'covgpu_check_immunity', 'covgpu_update_nab', 'covgpu_update_peak_nab',
             'covgpu_pop_scan_scratch'] + POP_FUNCS

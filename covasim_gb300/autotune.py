@@ -19,7 +19,7 @@ import numpy as np
 import torch
 
 from . import _lib as L
-from .sim import init_infections
+from .sim import init_infections_all
 from .state import parse_edge_tile
 
 __all__ = ['tune_edge_tile', 'workload_signature']
@@ -37,8 +37,7 @@ def workload_signature(state):
 
 def _one_run(state, snap, t1):
     state.restore(snap)
-    for k, sp in enumerate(state.specs):
-        init_infections(state, k, sp.pars)
+    init_infections_all(state, [sp.pars for sp in state.specs])
     state.run_days(0, t1, open_prev=False, close_last=True, use_graph=True)
 
 

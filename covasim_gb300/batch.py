@@ -17,7 +17,7 @@ from . import parameters as cvpar
 from . import immunity as cvimm
 from . import defaults as cvd
 from . import _lib as L
-from .sim import Sim, build_spec, init_infections, variant_import_count, CALL_IMPORT
+from .sim import Sim, build_spec, init_infections_all, variant_import_count, CALL_IMPORT
 from .state import BatchState
 
 __all__ = ['BatchSim']
@@ -71,8 +71,7 @@ class BatchSim:
         return self
 
     def seed_infections(self):
-        for k, s in enumerate(self.sims):
-            init_infections(self.state, k, s.pars)
+        init_infections_all(self.state, [s.pars for s in self.sims])
 
     def _import_variants(self, t):
         """Each sim's variant importations of day t, with the sim's own draws
@@ -80,10 +79,9 @@ class BatchSim:
         for k, s in enumerate(self.sims):
             for v in s['variants']:
                 if t in np.atleast_1d(v.days):
-                    sus = np.nonzero(self.state.get('susceptible', k).cpu().numpy())[0]
                     rng = np.random.default_rng([int(s['rand_seed']), 0x1A1A, t, v.index])
-                    n_imp = variant_import_count(v, self.state.rescale_vecs[k][t], rng)  # more than len(sus): ValueError
-                    inds = rng.choice(sus, n_imp, replace=False)
+                    n_imp = variant_import_count(v, self.state.rescale_vecs[k][t], rng)
+                    inds = self.state.choose_susceptible(k, n_imp, rng)  # more than there are: ValueError
                     self.state.set_hospicu([[0, 0]] * len(self.sims))  # variant.apply: no bed limits
                     self.state.infect_list(t, inds, sim=k, variant=v.index, layer_tag=L.LOG_IMPORT,
                                            call_tag=CALL_IMPORT + v.index)
@@ -128,7 +126,7 @@ class BatchSim:
 
     def series(self, key):
         """[n_sims, npts] array of one per-day result."""
-        return np.stack([self.state.results(k)[key] for k in range(len(self.sims))])
+        return self.state.series(key)
 
     def finalize(self):
         """Fill each Sim's results as Sim.finalize does."""

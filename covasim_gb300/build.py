@@ -16,7 +16,8 @@ CSRC = os.path.join(HERE, 'csrc')
 INCLUDE = os.path.join(ROOT, 'include')
 LIB_NAME = 'libcovgpu.so'
 LIB_PATH = os.path.join(HERE, LIB_NAME)
-SOURCES = ['covgpu.cu', 'covgpu_reference.cu', 'covgpu_testing.cu', 'covgpu_pop.cu', 'covgpu_dropin.cu']
+SOURCES = ['covgpu.cu', 'covgpu_reference.cu', 'covgpu_testing.cu', 'covgpu_pop.cu', 'covgpu_dropin.cu',
+           'covgpu_copy.cu']
 OBJ_DIR = os.path.join(HERE, '_build')
 ARCH = ['-gencode', 'arch=compute_103a,code=sm_103a']
 

@@ -2282,29 +2282,40 @@ __global__ void k_infect_list(covgpu_state st, int t, const int32_t* inds, const
 // stream CALL_TAG_IMPORT. The trip count is uniform across each block (the
 // ballots of infect_tally need every lane); lanes of one warp may belong to
 // different sims.
-__global__ void k_import_day(covgpu_state st, int t) {
-  if (held(st, t)) return;
-  const int64_t b = st.import_day_off[t], e = st.import_day_off[t + 1];
+__device__ __forceinline__ void infect_entries(const covgpu_state& st, int t, const int32_t* inds,
+                                               const int32_t* sims, int64_t b, int64_t e, int v, int layer_tag,
+                                               int call_tag) {
   for (int64_t base = b + (int64_t)blockIdx.x * blockDim.x; base < e; base += (int64_t)gridDim.x * blockDim.x) {
     const int64_t j = base + threadIdx.x;
     uint32_t out = 0;
     int32_t tgt = 0, s = 0;
     if (j < e) {
-      const int64_t i = st.imports[j];
-      s = st.import_sims[j];
+      const int64_t i = inds[j];
+      s = sims[j];
       if (s >= 0 && s < st.n_sims && i >= st.sims[s].agent_off && i < st.sims[s].agent_off + st.sims[s].n_agents) {
         const covgpu_sim_params& sp = st.sims[s];
         bool hosp, icu;
         hosp_icu(st, sp, s, t, hosp, icu);
         tgt = (int32_t)(i - sp.agent_off);
-        out = infect_one(st, sp, s, i, t, 0, -1, COVGPU_MAX_LAYERS + 1, CALL_TAG_IMPORT, hosp, icu);
+        out = infect_one(st, sp, s, i, t, v, -1, layer_tag, call_tag, hosp, icu);
       } else {
         atomicOr(st.status, COVGPU_BADARG);
         s = 0;
       }
     }
-    infect_tally(st, t, out, s, 0, -1, tgt, COVGPU_MAX_LAYERS + 1);
+    infect_tally(st, t, out, s, v, -1, tgt, layer_tag);
   }
+}
+__global__ void k_import_day(covgpu_state st, int t) {
+  if (held(st, t)) return;
+  infect_entries(st, t, st.imports, st.import_sims, st.import_day_off[t], st.import_day_off[t + 1], 0,
+                 COVGPU_MAX_LAYERS + 1, CALL_TAG_IMPORT);
+}
+// the agents of several sims at once (a batch's seed infections: one launch instead of
+// one and its uploads per sim)
+__global__ void k_infect_sims(covgpu_state st, int t, const int32_t* inds, const int32_t* sims, int64_t n, int v,
+                              int layer_tag, int call_tag) {
+  infect_entries(st, t, inds, sims, 0, n, v, layer_tag, call_tag);
 }
 
 // sim.py:535-547, the test only: is a rescaling due at the start of day t? The
@@ -2494,6 +2505,17 @@ int covgpu_infect_list(const covgpu_state* st, int32_t t, const int32_t* inds, c
   if (!inds) return COVGPU_BADARG;
   k_infect_list<<<grid_for(n_inds, 128), 128, 0, S(stream)>>>(*st, t, inds, sources, n_inds, sim, variant, layer_tag,
                                                                call_tag, infected);
+  return launch_status();
+}
+
+int covgpu_infect_sims(const covgpu_state* st, int32_t t, const int32_t* inds, const int32_t* sims, int64_t n_inds,
+                       int32_t variant, int32_t layer_tag, int32_t call_tag, void* stream) {
+  int rc = check_state(st);
+  if (rc) return rc;
+  if (t < 0 || t >= 0xFFFF || n_inds < 0 || variant < 0 || variant >= COVGPU_MAX_VARIANTS) return COVGPU_BADARG;
+  if (n_inds == 0) return COVGPU_OK;
+  if (!inds || !sims) return COVGPU_BADARG;
+  k_infect_sims<<<grid_for(n_inds, 128), 128, 0, S(stream)>>>(*st, t, inds, sims, n_inds, variant, layer_tag, call_tag);
   return launch_status();
 }
 

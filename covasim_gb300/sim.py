@@ -68,15 +68,16 @@ def mean_infectious_duration(d_rec, d_dead, d_inf):
     """sim.py:920-932: mean of the outcome dates minus mean of the infectious dates,
     over the agents with a recovery date then those with a death date (numpy
     arrays or device tensors; sums in float64)."""
-    if torch.is_tensor(d_rec):  # masked sums on the device, one read-back
-        m_rec, m_dead = ~torch.isnan(d_rec), ~torch.isnan(d_dead)
-        zero = d_rec.new_zeros(())
-        sums = torch.stack([m_rec.sum().double() + m_dead.sum().double(),
-                            torch.where(m_rec, d_rec, zero).double().sum() +
-                            torch.where(m_dead, d_dead, zero).double().sum(),
-                            torch.where(m_rec, d_inf, zero).double().sum() +
-                            torch.where(m_dead, d_inf, zero).double().sum()])
-        n_out, s_out, s_inf = sums.tolist()
+    if torch.is_tensor(d_rec) and not all(x.is_cuda and x.dtype == torch.float32 for x in (d_rec, d_dead, d_inf)):
+        d_rec, d_dead, d_inf = (x.cpu().numpy() for x in (d_rec, d_dead, d_inf))
+    if torch.is_tensor(d_rec):  # per-block sums on the device, one read-back
+        d_rec, d_dead, d_inf = (x.contiguous() for x in (d_rec, d_dead, d_inf))
+        if not d_rec.numel():
+            return 0.0
+        sums = torch.empty((L.OUTCOME_BLOCKS, 3), dtype=torch.float64, device=d_rec.device)
+        L.call('covgpu_outcome_sums', d_rec.data_ptr(), d_dead.data_ptr(), d_inf.data_ptr(), d_rec.numel(),
+               sums.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        n_out, s_out, s_inf = sums.cpu().numpy().sum(axis=0).tolist()
         if not n_out:
             return 0.0
     else:
@@ -219,6 +220,19 @@ def init_infections(state, k, pars):
         inds = choose_seed_infections(pars['rand_seed'], pars['pop_size'], pars['pop_infected'])
         state.infect_list(0, inds, sim=k, variant=0, layer_tag=L.LOG_SEED, call_tag=CALL_SEED)
     state.count_nonnaive(k)
+
+
+def init_infections_all(state, all_pars):
+    """``init_infections`` for every sim of a batch, the seed infections of all of
+    them in one launch."""
+    for k, pars in enumerate(all_pars):
+        if pars['frac_susceptible'] < 1:
+            state.make_nonnaive(choose_nonnaive(pars['rand_seed'], pars['pop_size'], pars['frac_susceptible']), sim=k)
+    state.infect_sims(0, [(k, choose_seed_infections(pars['rand_seed'], pars['pop_size'], pars['pop_infected']))
+                          for k, pars in enumerate(all_pars) if pars['pop_infected']],
+                      variant=0, layer_tag=L.LOG_SEED, call_tag=CALL_SEED)
+    for k in range(len(all_pars)):
+        state.count_nonnaive(k)
 
 
 def _layers_from_popdict(pars, popdict):
@@ -525,10 +539,9 @@ class Sim:
         """immunity.py:117-130 variant.apply: import n_imports agents chosen among the susceptible."""
         for v in self['variants']:
             if t in np.atleast_1d(v.days):
-                sus = np.nonzero(self.people['susceptible'])[0]
                 rng = np.random.default_rng([int(self['rand_seed']), 0x1A1A, t, v.index])
-                n_imp = variant_import_count(v, self.state.rescale_vecs[0][t], rng)  # more than len(sus): ValueError, as immunity.py:128
-                inds = rng.choice(sus, n_imp, replace=False)
+                n_imp = variant_import_count(v, self.state.rescale_vecs[0][t], rng)
+                inds = self.state.choose_susceptible(0, n_imp, rng)  # more than there are: ValueError, as immunity.py:128
                 self.state.set_hospicu([[0, 0]])  # variant.apply calls infect() without bed limits
                 self.state.infect_list(t, inds, sim=0, variant=v.index, layer_tag=L.LOG_IMPORT,
                                        call_tag=CALL_IMPORT + v.index)

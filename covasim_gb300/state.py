@@ -381,9 +381,10 @@ class BatchState:
         self.t = t
 
         # per-sim tables, concatenated
-        self.res_int = torch.zeros(sum(sp.npts for sp in self.specs) * L.N_RES_INT, dtype=I64, device=dev)
-        self.res_var = torch.zeros(sum(sp.npts * L.N_RES_VAR * sp.nv for sp in self.specs), dtype=I64, device=dev)
-        self.res_fx = torch.zeros(sum(sp.npts for sp in self.specs) * L.N_RES_F, dtype=I64, device=dev)
+        days = sum(sp.npts for sp in self.specs)
+        sizes = [days * L.N_RES_INT, sum(sp.npts * L.N_RES_VAR * sp.nv for sp in self.specs), days * L.N_RES_F]
+        self.res_all = torch.zeros(sum(sizes), dtype=I64, device=dev)  # one buffer: read back and cleared at once
+        self.res_int, self.res_var, self.res_fx = self.res_all.split(sizes)
         beta_tabs, bl_tabs, kins = [], [], []
         for sp in self.specs:
             beta_tabs.append(sp.beta_table().ravel())
@@ -1038,8 +1039,7 @@ class BatchState:
         self.lik['factor'][sim, :T, :Lm, :V].copy_(pair)
 
     def zero_lik(self):
-        for k in ('ll', 'expected', 'g_ll', 'g_exp', 'logq', 'w'):
-            self.lik[k].zero_()
+        self._spans([], [self.lik[k] for k in ('ll', 'expected', 'g_ll', 'g_exp', 'logq', 'w')])
 
     def lik_targets(self, t):
         """Per-target half of day t's likelihood (after edge_pass, before infect_claims)."""
@@ -1124,6 +1124,28 @@ class BatchState:
                                      infected, self.t['status'])
         return (inds, infected) if want_infected else None
 
+    def choose_susceptible(self, sim, n, rng):
+        """``rng.choice(susceptible, n, replace=False)`` over the local indices of one
+        sim's susceptible agents, which stay on the device."""
+        sus = torch.nonzero(self.t['flags'][self.sl(sim)] & (1 << STATE_BIT['susceptible'])).squeeze(1)
+        pick = torch.from_numpy(rng.choice(len(sus), n, replace=False))
+        return sus[pick.to(self.device)].cpu().numpy()
+
+    def infect_sims(self, t, lists, variant=0, layer_tag=L.LOG_SEED, call_tag=1):
+        """Infect explicit agents of several sims in one launch: ``lists`` of (sim,
+        distinct local indices)."""
+        lists = [(k, np.asarray(inds, dtype=np.int64)) for k, inds in lists if len(inds)]
+        if not lists:
+            return
+        for k, inds in lists:
+            if inds.min() < 0 or inds.max() >= self.specs[k].n:
+                raise IndexError('agent index out of range')
+        both = np.stack([np.concatenate([inds + self.offsets[k] for k, inds in lists]),
+                         np.repeat([k for k, _ in lists], [len(inds) for _, inds in lists])]).astype(np.int32)
+        inds, sims = self._keep_inds = _upload(both, self.device).unbind()
+        torch.ops.covgpu.infect_sims(self._sa, int(t), inds, sims, int(variant), int(layer_tag), int(call_tag),
+                                     self.t['status'])
+
     def run_days(self, t0, t1, open_prev=False, close_last=True, use_graph=True):
         torch.ops.covgpu.run_days(self._sa, int(t0), int(t1), bool(open_prev), bool(close_last), bool(use_graph),
                                   self.t['status'])
@@ -1195,25 +1217,37 @@ class BatchState:
         keys = self.MUTABLE + (('pending_quar',) if self.has_testing else ())
         return {k: self.t[k].clone() for k in keys}
 
+    def _spans(self, copies, zeros=(), ones=()):
+        """Copy each (dst, src) pair, zero each of ``zeros`` and set every bit of each
+        of ``ones`` in one launch (covgpu_copy_spans); pairs that are not plain
+        copies (another type, size, layout or device) go through ``copy_``."""
+        todo, dev = [], self.res_all.device
+        for dst, src in copies:
+            if (type(src) is torch.Tensor and src.dtype == dst.dtype and src.shape == dst.shape and
+                    src.device == dev and dst.is_contiguous() and src.is_contiguous()):
+                todo.append((dst, src.data_ptr(), 0))
+            else:
+                dst.copy_(src)
+        todo += [(x, None, 0) for x in zeros] + [(x, None, 0xFF) for x in ones]
+        spans = (L.Span * len(todo))(*((x.data_ptr(), src, x.numel() * x.element_size(), fill, 0)
+                                       for x, src, fill in todo))
+        L.call('covgpu_copy_spans', spans, len(todo), _stream())
+
+    def _day_buffers(self):
+        """The day-local buffers a rewind clears: (zeroed, all bits set)."""
+        t = self.t
+        keys = ('event_count', 'status') + (('trace_bits', 'contact_bits', 'trace_count') if self.has_testing else ())
+        return [t[k] for k in keys], [t['claim']]
+
     def restore(self, snap):
         """Rewind to a snapshot: agent arrays, results, claims, counters and status."""
-        for k, v in snap.items():
-            self.t[k].copy_(v)
-        self.res_int.zero_()
-        self.res_var.zero_()
-        self.res_fx.zero_()
-        self.t['claim'].fill_(-1)
-        self.t['roles'].zero_()
-        self.t['viral_load'].zero_()
-        self.t['event_count'].zero_()
-        self.t['log_count'].zero_()
-        self.t['status'].zero_()
+        t = self.t
+        zeros, ones = self._day_buffers()
+        self._spans([(t[k], v) for k, v in snap.items()],
+                    zeros + [self.res_all, t['roles'], t['viral_load'], t['log_count']], ones)
         for a in self.import_variant:
             a[:] = 0
         self._reset_rescale()
-        if self.has_testing:
-            for k in ('trace_bits', 'contact_bits', 'trace_count'):
-                self.t[k].zero_()
         self._refresh_state()
 
     def checkpoint(self, into=None):
@@ -1222,11 +1256,9 @@ class BatchState:
         an earlier checkpoint of this state whose buffers are overwritten (no
         allocation)."""
         keys = self.MUTABLE + (('pending_quar',) if self.has_testing else ()) + ('log_count',)
+        res = (self.res_int, self.res_var, self.res_fx)
         if into is not None:
-            for k in keys:
-                into[k].copy_(self.t[k])
-            for dst, src in zip(into['_res'], (self.res_int, self.res_var, self.res_fx)):
-                dst.copy_(src)
+            self._spans([(into[k], self.t[k]) for k in keys] + list(zip(into['_res'], res)))
             for a, b in zip(into['_imp'], self.import_variant):
                 a[:] = b
             return into
@@ -1237,19 +1269,11 @@ class BatchState:
 
     def rewind(self, ck):
         """Return to a checkpoint (day-local buffers cleared, claims reset)."""
-        for k, v in ck.items():
-            if k not in ('_res', '_imp'):
-                self.t[k].copy_(v)
+        zeros, ones = self._day_buffers()
+        self._spans([(self.t[k], v) for k, v in ck.items() if k not in ('_res', '_imp')] +
+                    list(zip((self.res_int, self.res_var, self.res_fx), ck['_res'])), zeros, ones)
         for a, b in zip(self.import_variant, ck['_imp']):
             a[:] = b
-        for dst, src in zip((self.res_int, self.res_var, self.res_fx), ck['_res']):
-            dst.copy_(src)
-        self.t['claim'].fill_(-1)
-        self.t['event_count'].zero_()
-        self.t['status'].zero_()
-        if self.has_testing:
-            for k in ('trace_bits', 'contact_bits', 'trace_count'):
-                self.t[k].zero_()
 
     def status(self):
         return int(self.t['status'].item())
@@ -1346,14 +1370,36 @@ class BatchState:
         else:
             raise KeyError(f'Key "{key}" cannot be set')
 
-    def results(self, sim=0):
-        """Per-day results of one sim as float64 numpy arrays, keyed like sim.results."""
+    def read_results(self):
+        """Every sim's results on the host, in one copy: (res_int, res_var, res_fx)."""
+        host = self.res_all.cpu()
+        return [x.numpy() for x in host.split([self.res_int.numel(), self.res_var.numel(), self.res_fx.numel()])]
+
+    def series(self, key):
+        """[n_sims, npts] float64 array of one per-day result (sims of the same length)."""
+        host = self.read_results()
+        if key in cvd.RES_INT_KEYS:
+            col = list(cvd.RES_INT_KEYS).index(key)
+            return np.stack([host[0][ri + col:ri + sp.npts * L.N_RES_INT:L.N_RES_INT].astype(np.float64)
+                             for (ri, _, _), sp in zip(self.res_slices, self.specs)])
+        return np.stack([self.results(k, host)[key] for k in range(len(self.specs))])
+
+    def results(self, sim=0, host=None):
+        """Per-day results of one sim as float64 numpy arrays, keyed like sim.results
+        (host: from a ``read_results`` of every sim)."""
         sp = self.specs[sim]
         ri, rv, rf = self.res_slices[sim]
         npts, nv = sp.npts, sp.nv
-        ints = self.res_int[ri:ri + npts * L.N_RES_INT].view(npts, L.N_RES_INT).cpu().numpy().astype(np.float64)
-        var = self.res_var[rv:rv + npts * L.N_RES_VAR * nv].view(npts, L.N_RES_VAR, nv).cpu().numpy().astype(np.float64)
-        fx = self.res_fx[rf:rf + npts * L.N_RES_F].view(npts, L.N_RES_F).cpu().numpy()
+        n_int, n_var, n_fx = npts * L.N_RES_INT, npts * L.N_RES_VAR * nv, npts * L.N_RES_F
+        if host is None:  # this sim's part alone of a batch
+            host = self.read_results() if len(self.specs) == 1 else [
+                x[o:o + m].cpu().numpy() for x, o, m in ((self.res_int, ri, n_int), (self.res_var, rv, n_var),
+                                                         (self.res_fx, rf, n_fx))]
+            if len(self.specs) > 1:
+                ri = rv = rf = 0
+        ints = host[0][ri:ri + n_int].reshape(npts, L.N_RES_INT).astype(np.float64)
+        var = host[1][rv:rv + n_var].reshape(npts, L.N_RES_VAR, nv).astype(np.float64)
+        fx = host[2][rf:rf + n_fx].reshape(npts, L.N_RES_F)
         out = {}
         for k, key in enumerate(cvd.RES_INT_KEYS):
             out[key] = ints[:, k]

@@ -74,6 +74,14 @@ def infect_list(state: int, t: int, inds: torch.Tensor, sources: Optional[torch.
            int(layer_tag), int(call_tag), _p(infected), _stream())
 
 
+@torch.library.custom_op('covgpu::infect_sims', mutates_args=('status',))
+def infect_sims(state: int, t: int, inds: torch.Tensor, sims: torch.Tensor, variant: int, layer_tag: int,
+                call_tag: int, status: torch.Tensor) -> None:
+    """covgpu_infect_sims: People.infect for explicit agents of several sims (people.py:435-586)."""
+    L.call('covgpu_infect_sims', _st(state), int(t), _p(inds), _p(sims), inds.numel(), int(variant), int(layer_tag),
+           int(call_tag), _stream())
+
+
 @torch.library.custom_op('covgpu::import_day', mutates_args=('status',))
 def import_day(state: int, t: int, status: torch.Tensor) -> None:
     """covgpu_import_day: the day's Poisson importations (sim.py:582-587)."""

@@ -595,6 +595,12 @@ int covgpu_infect_list(const covgpu_state* st, int32_t t, const int32_t* inds, c
                        int32_t sim, int32_t variant, int32_t layer_tag, int32_t call_tag, uint8_t* infected,
                        void* stream);
 
+/* The same for agents of several sims in one launch: inds[j] (global, unique) is
+ * an agent of sim sims[j]; no sources are recorded. Entries outside their sim's
+ * agents are skipped and set COVGPU_BADARG in the device status word. */
+int covgpu_infect_sims(const covgpu_state* st, int32_t t, const int32_t* inds, const int32_t* sims, int64_t n_inds,
+                       int32_t variant, int32_t layer_tag, int32_t call_tag, void* stream);
+
 /* The day's importations (sim.py:582-587): infect() with the wild type for the
  * agents st->imports lists for day t (all sims; infection log layer
  * COVGPU_MAX_LAYERS + 1, Philox stream call_tag 2). covgpu_run_days runs it
@@ -631,6 +637,30 @@ int covgpu_layer_lists(const covgpu_state* st, int32_t segment, int32_t t, int64
  * directly (a run made once does not pay for the capture). */
 int covgpu_run_days(const covgpu_state* st, int32_t t0, int32_t t1, int32_t open_prev, int32_t close_last,
                     int32_t use_graph, void* stream);
+
+/* ---- whole-state copies and a run's outcome sums ------------------------ */
+
+/* One array of a covgpu_copy_spans call: src's bytes into dst, or, with src
+ * NULL, every byte of dst set to fill. */
+typedef struct covgpu_span {
+  void* dst;
+  const void* src;
+  int64_t bytes;
+  int32_t fill;
+  int32_t _pad;
+} covgpu_span;
+
+/* Copy or fill n device arrays (spans: a host array, read before the call
+ * returns) in one launch per 40. No span may overlap another's dst. */
+int covgpu_copy_spans(const covgpu_span* spans, int32_t n, void* stream);
+
+/* sim.py:920-932 (compute_r_eff's mean infectious duration): COVGPU_OUTCOME_BLOCKS
+ * partial sums out[b][3] over n agents: agents with a recovery date plus agents
+ * with a death date, the sum of those dates, the sum of the infectious dates of
+ * the same agents. */
+#define COVGPU_OUTCOME_BLOCKS 304
+int covgpu_outcome_sums(const float* date_recovered, const float* date_dead, const float* date_infectious, int64_t n,
+                        double* out, void* stream);
 
 /* ---- the day path one function at a time --------------------------------
  * For callers that keep the reference's call sequence (update_states_pre's
