@@ -102,6 +102,7 @@ class SimParams(C.Structure):
         ('testing', Testing), ('seg_of_layer', C.c_int32 * MAX_LAYERS),
         ('pop_scale', C.c_double), ('rescale_threshold', C.c_double), ('rescale_vec', C.c_void_p),
         ('nonnaive', C.c_void_p),
+        ('dur_ff', (C.c_float * 4) * (len(DUR_ORDER) + 1)), ('dur_int', C.c_int32), ('_pad3', C.c_int32),
     ]
 
 

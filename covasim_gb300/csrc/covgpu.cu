@@ -1976,7 +1976,6 @@ __device__ uint32_t infect_group(const covgpu_state& st, const covgpu_sim_params
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31, r = lane & (IG - 1), g0 = lane & ~(IG - 1);
   const uint32_t f0 = win ? st.flags[i] : 0u;
-  const bool act = win && (f0 & B_SUS);  // people.py:468-472: keep only susceptibles
   const int64_t local = i - sp.agent_off;
   const bool injected = st.draw_table != nullptr;
   const double* tab = injected ? st.draw_table + i * COVGPU_N_DRAWS : nullptr;
@@ -2001,16 +2000,31 @@ __device__ uint32_t infect_group(const covgpu_state& st, const covgpu_sim_params
     a_nbt = st.n_breakthroughs[i];
     a_rt = st.rel_trans[i];
   }
-  // the branch: every lane of the group (people.py:523-566)
-  bool symp = false, sev = false, crit = false, dead = false;
-  uint4 b1 = make_uint4(0u, 0u, 0u, 0u);
-  if (act) {
-    uint32_t uw[4] = {0u, 0u, 0u, 0u};
-    if (!injected) {
-      b1 = philox(make_uint4((uint32_t)local, 1u, (uint32_t)t, tag), sp.key0, sp.key1);
+  // This lane's normals, in converged code (every lane of a group runs the same Philox
+  // and Box-Muller instructions on its own inputs) and before the loaded fields are
+  // used, so that their latency is covered. Lane 0: z0, z1; lane 1: z2, z3; lanes 2
+  // and 3: z4, z5.
+  uint32_t uw[4] = {0u, 0u, 0u, 0u};
+  ff za{0.0f, 0.0f}, zb{0.0f, 0.0f};
+  if (win) {
+    if (injected) {
+      const int k = 2 * (r < 2 ? r : 2);
+      za = d2ff(tab[k]);
+      zb = d2ff(tab[k + 1]);
+    } else {
+      const uint4 b0 = philox(make_uint4((uint32_t)local, 0u, (uint32_t)t, tag), sp.key0, sp.key1);
+      const uint4 b1 = philox(make_uint4((uint32_t)local, 1u, (uint32_t)t, tag), sp.key0, sp.key1);
       const uint4 b2 = philox(make_uint4((uint32_t)local, 2u, (uint32_t)t, tag), sp.key0, sp.key1);
       uw[0] = b1.z; uw[1] = b1.w; uw[2] = b2.x; uw[3] = b2.y;
+      const uint32_t wa = r == 0 ? b0.x : (r == 1 ? b0.z : b1.x);
+      const uint32_t wb = r == 0 ? b0.y : (r == 1 ? b0.w : b1.y);
+      box_muller_ff(wa, wb, COVGPU_LN_TAB, COVGPU_LN_INV, COVGPU_SINCOS_TAB, za, zb);
     }
+  }
+  const bool act = win && (f0 & B_SUS);  // people.py:468-472: keep only susceptibles
+  // the branch: every lane of the group (people.py:523-566)
+  bool symp = false, sev = false, crit = false, dead = false;
+  if (act) {
     auto lt = [&](int k, float p) { return injected ? (tab[6 + k] < (double)p) : bern32(uw[k], p); };
     // symp_imm as symp_imm_of reads it: 0 for an agent that never had NAbs
     const float sp_symp = __fmul_rn(__fmul_rn(sp.rel_symp[v], a_symp), __fsub_rn(1.0f, a_peak == 0.0f ? 0.0f : a_simm));
@@ -2029,47 +2043,50 @@ __device__ uint32_t infect_group(const covgpu_state& st, const covgpu_sim_params
       }
     }
   }
-  // This lane's normals and samples, in converged code: every lane of an acting
-  // group runs the same Philox, Box-Muller and sampler instructions on its own
-  // inputs (divergent per-lane branches would run one after another).
-  // Lane 0: exp2inf, inf2sym (normals z0, z1); lane 1: sym2sev, sev2crit (z2, z3);
-  // lane 2: the recovery or death duration (z4); lane 3: the initial NAb (z5).
+  // The samples: lane 0 exp2inf and inf2sym, lane 1 sym2sev and sev2crit, lane 2 the
+  // recovery or death duration, lane 3 the initial NAb (first sample of every lane;
+  // the second of lanes 0 and 1, the others repeat a harmless one to stay converged).
+  // With dur_int every lane runs one exponential per sample, lane 3's of its level
+  // times ln 2, and days are whole float32 numbers: no float64 but lane 3's level.
+  const bool days = act && sp.dur_int && !injected;  // injected draws keep the general form's pairs
   double s0 = 0.0, s1 = 0.0;
-  float peak = 0.0f;
+  float f_0 = 0.0f, f_1 = 0.0f, peak = 0.0f;
   if (act) {
-    ff za, zb;
-    if (injected) {
-      const int k = 2 * (r < 2 ? r : 2);
-      za = d2ff(tab[k]);
-      zb = d2ff(tab[k + 1]);
-    } else {
-      const uint4 b0 = philox(make_uint4((uint32_t)local, 0u, (uint32_t)t, tag), sp.key0, sp.key1);
-      const uint32_t wa = r == 0 ? b0.x : (r == 1 ? b0.z : b1.x);
-      const uint32_t wb = r == 0 ? b0.y : (r == 1 ? b0.w : b1.y);
-      box_muller_ff(wa, wb, COVGPU_LN_TAB, COVGPU_LN_INV, COVGPU_SINCOS_TAB, za, zb);
-    }
     const int rec_d = !symp ? COVGPU_D_ASYM2REC : (!sev ? COVGPU_D_MILD2REC : (!crit ? COVGPU_D_SEV2REC
                                                                                 : (dead ? COVGPU_D_CRIT2DIE
                                                                                         : COVGPU_D_CRIT2REC)));
-    // first sample of every lane; the second of lanes 0 and 1 (the others repeat a
-    // harmless one to stay converged)
-    const covgpu_dur_par& p0 = r == 0 ? sp.dur[COVGPU_D_EXP2INF]
-                                      : (r == 1 ? sp.dur[COVGPU_D_SYM2SEV] : (r == 2 ? sp.dur[rec_d] : sp.nab_init));
-    const covgpu_dur_par& p1 = r == 0 ? sp.dur[COVGPU_D_INF2SYM] : (r == 1 ? sp.dur[COVGPU_D_SEV2CRIT] : p0);
-    s0 = sample_ff(p0, r == 3 ? zb : za);
-    s1 = sample_ff(p1, r < 2 ? zb : (r == 3 ? zb : za));
+    const int k0 = r == 0 ? COVGPU_D_EXP2INF : (r == 1 ? COVGPU_D_SYM2SEV : (r == 2 ? rec_d : COVGPU_N_DUR_PARS));
+    const int k1 = r == 0 ? COVGPU_D_INF2SYM : (r == 1 ? COVGPU_D_SEV2CRIT : k0);
+    double level = 0.0;  // lane 3: 2^(initial NAb)
+    if (days) {
+      const float* p0 = sp.dur_ff[k0];
+      const float* p1 = sp.dur_ff[k1];
+      ff y0 = ff_add(ff{p0[0], p0[1]}, ff_mul(ff{p0[2], p0[3]}, r == 3 ? zb : za));
+      const ff y1 = ff_add(ff{p1[0], p1[1]}, ff_mul(ff{p1[2], p1[3]}, r < 2 ? zb : za));
+      if (r == 3) y0 = ff_mul(d2ff(ff2d(y0)), ff{COVGPU_LN2_FF_HI, COVGPU_LN2_FF_LO});  // exp2_ff of the stored float64
+      const ff e0 = ff_exp_uniform(y0, COVGPU_EXP_TAB), e1 = ff_exp_uniform(y1, COVGPU_EXP_TAB);
+      f_0 = ff_rint(e0);
+      f_1 = ff_rint(e1);
+      if (r == 3) level = ff2d(e0);
+    } else {
+      const covgpu_dur_par& p0 = r < 3 ? sp.dur[k0] : sp.nab_init;
+      const covgpu_dur_par& p1 = r < 2 ? sp.dur[k1] : p0;
+      s0 = sample_ff(p0, r == 3 ? zb : za);
+      s1 = sample_ff(p1, r < 2 ? zb : (r == 3 ? zb : za));
+      f_0 = (float)s0;
+      f_1 = (float)s1;
+      if (r == 3 && sp.use_waning) level = exp2_ff(d2ff(s0));
+    }
     if (r == 3 && sp.use_waning) {  // immunity.py:138-202 update_peak_nab (natural infection)
-      if (a_nab > 0.0f) {
-        peak = __fmul_rn(a_peak, sp.nab_boost);
-      } else {
-        const double rel = !symp ? sp.rel_imm_asymp : (!sev ? sp.rel_imm_mild : sp.rel_imm_severe);
-        peak = (float)__dmul_rn(__dmul_rn(exp2_ff(d2ff(s0)), rel), sp.nab_norm);
-      }
+      const double rel = !symp ? sp.rel_imm_asymp : (!sev ? sp.rel_imm_mild : sp.rel_imm_severe);
+      peak = a_nab > 0.0f ? __fmul_rn(a_peak, sp.nab_boost) : (float)__dmul_rn(__dmul_rn(level, rel), sp.nab_norm);
     }
   }
-  const double v_exp2inf = __shfl_sync(full, s0, g0), v_inf2sym = __shfl_sync(full, s1, g0);
-  const double v_sym2sev = __shfl_sync(full, s0, g0 + 1), v_sev2crit = __shfl_sync(full, s1, g0 + 1);
-  const double v_rec = __shfl_sync(full, s0, g0 + 2);
+  const float v_exp2inf = __shfl_sync(full, f_0, g0), v_inf2sym = __shfl_sync(full, f_1, g0);
+  const float v_sym2sev = __shfl_sync(full, f_0, g0 + 1), v_sev2crit = __shfl_sync(full, f_1, g0 + 1);
+  const float v_days = __shfl_sync(full, f_0, g0 + 2);
+  double v_rec = 0.0;
+  if (__any_sync(full, act && !days)) v_rec = __shfl_sync(full, s0, g0 + 2);
   const float v_peak = __shfl_sync(full, peak, g0 + 3);
   if (r != 0 || !act) return 0u;
 
@@ -2094,7 +2111,7 @@ __device__ uint32_t infect_group(const covgpu_state& st, const covgpu_sim_params
   float* u_disease = dur_row(st, COVGPU_DUR_DISEASE);
   const float nanf_ = f32nan();
   const float tf = (float)t;
-  const float de = (float)v_exp2inf;  // people.py:514-520
+  const float de = v_exp2inf;  // people.py:514-520
   dur_row(st, COVGPU_DUR_EXP2INF)[i] = de;
   date_row(st, COVGPU_DATE_EXPOSED)[i] = tf;
   const float di = __fadd_rn(de, tf);
@@ -2102,40 +2119,41 @@ __device__ uint32_t infect_group(const covgpu_state& st, const covgpu_sim_params
   d_sym[i] = nanf_; d_sev[i] = nanf_; d_crit[i] = nanf_;
   date_row(st, COVGPU_DATE_DIAGNOSED)[i] = nanf_;
   float rec = nanf_;
-  const double dr = v_rec;
+  // x plus the recovery or death duration, rounded once (whole days: exact in float32)
+  auto plus = [&](float x) { return days ? __fadd_rn(x, v_days) : (float)__dadd_rn((double)x, v_rec); };
   if (!symp) {  // CASE 1: asymptomatic, people.py:530-532
-    rec = (float)__dadd_rn((double)di, dr);
-    u_disease[i] = (float)__dadd_rn((double)de, dr);
+    rec = plus(di);
+    u_disease[i] = plus(de);
   } else {  // CASE 2: symptomatic, people.py:535-541
-    const float dis = (float)v_inf2sym;
+    const float dis = v_inf2sym;
     dur_row(st, COVGPU_DUR_INF2SYM)[i] = dis;
     const float ds = __fadd_rn(di, dis);
     d_sym[i] = ds;
     out |= O_SYMP;
     if (!sev) {  // CASE 2.1 mild, people.py:544-547
-      rec = (float)__dadd_rn((double)ds, dr);
-      u_disease[i] = (float)__dadd_rn((double)__fadd_rn(de, dis), dr);
+      rec = plus(ds);
+      u_disease[i] = plus(__fadd_rn(de, dis));
     } else {  // CASE 2.2 severe, people.py:550-554
       out |= O_SEV;
-      const float dss = (float)v_sym2sev;
+      const float dss = v_sym2sev;
       dur_row(st, COVGPU_DUR_SYM2SEV)[i] = dss;
       const float dsev = __fadd_rn(ds, dss);
       d_sev[i] = dsev;
       if (!crit) {  // CASE 2.2.1 not critical, people.py:557-559
-        rec = (float)__dadd_rn((double)dsev, dr);
-        u_disease[i] = (float)__dadd_rn((double)__fadd_rn(__fadd_rn(de, dis), dss), dr);
+        rec = plus(dsev);
+        u_disease[i] = plus(__fadd_rn(__fadd_rn(de, dis), dss));
       } else {  // CASE 2.2.2 critical, people.py:562-566
-        const float dsc = (float)v_sev2crit;
+        const float dsc = v_sev2crit;
         dur_row(st, COVGPU_DUR_SEV2CRIT)[i] = dsc;
         const float dcrit = __fadd_rn(dsev, dsc);
         d_crit[i] = dcrit;
         const float dsum = __fadd_rn(__fadd_rn(__fadd_rn(de, dis), dss), dsc);
         if (!dead) {  // CASE 2.2.2.1 alive, people.py:569-571
-          rec = (float)__dadd_rn((double)dcrit, dr);
-          u_disease[i] = (float)__dadd_rn((double)dsum, dr);
+          rec = plus(dcrit);
+          u_disease[i] = plus(dsum);
         } else {  // CASE 2.2.2.2 dead, people.py:574-577
-          d_dead[i] = (float)__dadd_rn((double)dcrit, dr);
-          u_disease[i] = (float)__dadd_rn((double)dsum, dr);
+          d_dead[i] = plus(dcrit);
+          u_disease[i] = plus(dsum);
         }
       }
     }
@@ -2219,7 +2237,22 @@ __device__ __forceinline__ void hosp_icu(const covgpu_state& st, const covgpu_si
   icu = sp.n_beds_icu >= 0 && r[COVGPU_RES_CRITICAL_NOW] > sp.n_beds_icu;
 }
 
+// loads one word of each 128-byte line of p[0, bytes), spread over the block's threads
+__device__ __forceinline__ void warm_l1(const void* p, size_t bytes) {
+  for (size_t k = 128 * threadIdx.x; k < bytes; k += 128 * blockDim.x) {
+    uint32_t x;
+    asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(x) : "l"(static_cast<const char*>(p) + k));
+  }
+}
+
 __global__ void k_infect_claims(covgpu_state st, int t) {
+  // the tables of the draws into L1 while the predecessor finishes (read-only; each
+  // infection would otherwise wait for them in turn)
+  warm_l1(&COVGPU_LN_TAB[0][0], sizeof(COVGPU_LN_TAB));
+  warm_l1(COVGPU_LN_INV, sizeof(COVGPU_LN_INV));
+  warm_l1(&COVGPU_SINCOS_TAB[0][0], sizeof(COVGPU_SINCOS_TAB));
+  warm_l1(&COVGPU_EXP_TAB[0][0], sizeof(COVGPU_EXP_TAB));
+  if (st.n_sims == 1) warm_l1(st.sims, sizeof(covgpu_sim_params));
   pdl_wait();
   pdl_trigger();  // the next day's agent pass may set up while the infections run
   if (held(st, t)) return;

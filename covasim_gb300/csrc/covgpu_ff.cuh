@@ -130,6 +130,17 @@ __device__ __forceinline__ ff ff_exp(ff y, const float (*tab)[2]) {
   return ff_div(ff{1.0f, 0.0f}, ff_exp_neg(ff{-y.hi, -y.lo}, tab));
 }
 
+// ff_exp without divergence: lanes with y of either sign run the same instructions
+// (the exponential of -|y| and its reciprocal) and select; the same bits as ff_exp
+__device__ __forceinline__ ff ff_exp_uniform(ff y, const float (*tab)[2]) {
+  const bool pos = !(y.hi <= 0.0f);
+  const ff x = ff_exp_neg(pos ? ff{-y.hi, -y.lo} : y, tab);
+  const ff r = ff_div(ff{1.0f, 0.0f}, x);
+  if (y.hi < -87.0f) return ff{0.0f, 0.0f};
+  if (y.hi > 87.0f) return ff{__int_as_float(0x7f800000), 0.0f};
+  return pos ? r : x;
+}
+
 // ln of a positive float-float: ln(hi) + lo / hi (|lo / hi| <= 2^-24, so the
 // dropped term is below 2^-49; lo / hi as lo times the reciprocal of hi)
 __device__ __forceinline__ ff ff_log_ff(ff x, const float (*tab)[2], const float* inv) {

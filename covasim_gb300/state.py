@@ -877,6 +877,11 @@ class BatchState:
                 r.dur[j] = dur_par(p['dur'][key])
             nab_init = p['nab_init']
             r.nab_init = dur_par(nab_init) if nab_init is not None else L.DurPar(L.DIST_ZERO, 0, 0.0, 0.0)
+            dists = [*r.dur, r.nab_init]
+            for d, pair in zip(dists, r.dur_ff):
+                pair[:] = (*ff_split(d.a), *ff_split(d.b))
+            r.dur_int = int(all(d.code == L.DIST_CODES['lognormal_int'] for d in r.dur) and
+                            r.nab_init.code in (L.DIST_CODES['normal'], L.DIST_ZERO if not r.use_waning else -1))
             r.nab_kin = self.nab_kin.data_ptr() + 4 * kn
             r.beta_tab = self.beta_tab.data_ptr() + 4 * bt
             r.beta_layer_tab = self.beta_layer_tab.data_ptr() + 4 * bl

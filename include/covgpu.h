@@ -210,6 +210,12 @@ typedef struct covgpu_sim_params {
   const double* rescale_vec;      /* [npts] current scale of each day               */
   int64_t* nonnaive;              /* [3] agents not naive, the last day whose flows
                                      are in that count, the last day checked        */
+  /* dur and nab_init once more as float pairs (a hi, a lo, b hi, b lo), read when
+   * dur_int is set: every duration is COVGPU_DIST_LOGNORMAL_INT and nab_init
+   * COVGPU_DIST_NORMAL (or unused), so that infect() needs no float64 for its days */
+  float dur_ff[COVGPU_N_DUR_PARS + 1][4];
+  int32_t dur_int;
+  int32_t _pad3;
 } covgpu_sim_params;
 
 /* One contact layer of one sim (device memory, one entry per layer segment).
