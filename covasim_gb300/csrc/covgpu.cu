@@ -54,6 +54,17 @@ constexpr int IMPORT_BLOCKS = 4;       // k_import_day grid (a day imports a han
 // ============================================================ fused agent pass
 
 
+// Fixed-point terms of the levels' sums, by 32-bit conversions (64-bit ones run at
+// the float64 rate, 16 cycles a warp): x * 2^24 of a NAb level (at least 128: the
+// 64-bit conversion), and x * 2^32 of an efficacy in [0, 1] (1 saturates).
+__device__ __forceinline__ long long nab_fixed(float x) {
+  const float y = __fmul_rn(x, 16777216.0f);
+  return y < 2147483648.0f ? (long long)__float2int_rn(y) : __float2ll_rn(y);
+}
+__device__ __forceinline__ long long efficacy_fixed(float x) {
+  return (long long)__float2uint_rn(__fmul_rn(x, 4294967296.0f)) + (x >= 1.0f ? 1 : 0);
+}
+
 // One agent's inputs that (nearly) every agent needs: the state words, rel_sus, the
 // recovery date and the NAb fields, loaded one agent block ahead of its processing.
 struct AgentIn {
@@ -134,10 +145,8 @@ __device__ __forceinline__ void ve_agent(const covgpu_state& st, const covgpu_si
     if (rs & 0x7FFFFFFFu)
       st.tgt_rec[off] = __uint_as_float(__float_as_uint(__fmul_rn(__uint_as_float(rs & 0x7FFFFFFFu),
                                                                   __fsub_rn(1.0f, a))) | (rs & 0x80000000u));
-    if (a != 0.0f || b != 0.0f) {
-      sus_fx += __float2ll_rn(__fmul_rn(a, 4294967296.0f));
-      symp_fx += __float2ll_rn(__fmul_rn(b, 4294967296.0f));
-    }
+    sus_fx += efficacy_fixed(a);
+    symp_fx += efficacy_fixed(b);
   }
 }
 
@@ -215,7 +224,7 @@ __device__ __forceinline__ void agent_block_step(const covgpu_state& st, const c
           nab_now = nab;
         }
       }
-      if (!(f & B_DEAD) && nab != 0.0f) nab_fx += __float2ll_rn(__fmul_rn(nab, 16777216.0f));  // sim.py:672
+      if (!(f & B_DEAD)) nab_fx += nab_fixed(nab);  // sim.py:672
     }
   }
 
