@@ -176,7 +176,7 @@ __device__ __forceinline__ void agent_block_step(const covgpu_state& st, const c
                                                  const AgentIn& in, int t, int do_prev, int do_day, int full_imm,
                                                  int steady, VeQueue& vq, int& qn,
                                                  const float (*s_ln_tab)[2], const float* s_ln_inv,
-                                                 const float (*s_exp_tab)[2],
+                                                 const float (*s_exp_tab)[2], const float* s_vl,
                                                  long long& nab_fx, long long& sus_fx, long long& symp_fx,
                                                  unsigned& acc_prev, unsigned& acc_day) {
   const covgpu_sim_params& sp = st.sims[blk.sim];
@@ -339,7 +339,7 @@ __device__ __forceinline__ void agent_block_step(const covgpu_state& st, const c
       // per endpoint instead of one per field)
       if (f & B_INF) {
         const float rt = a_rt;
-        const float vl = viral_load_one(t, d_inf, a_dr, d_dead, sp.frac_time, sp.load_ratio, sp.high_cap);
+        const float vl = s_vl[viral_load_early(t, d_inf, a_dr, d_dead, sp.frac_time, sp.high_cap) ? 1 : 0];
         st.viral_load[i] = vl;
         src_bit = (rt != 0.0f && iv < (uint32_t)nv) ? 1u : 0u;
         if (src_bit)
@@ -489,6 +489,8 @@ __global__ void __launch_bounds__(AGENT_THREADS, QUEUE ? AGENT_QUEUE_BLOCKS : AG
   agent_counters_clear(sc);
   covgpu_agent_block blk = st.agent_blocks[b];
   int sim = blk.sim;
+  __shared__ float s_vl[2];  // the sim's low and high viral loads
+  if (threadIdx.x < 2) s_vl[threadIdx.x] = viral_load_of(threadIdx.x == 1, st.sims[sim].frac_time, st.sims[sim].load_ratio);
   __syncthreads();
 
   pdl_wait();
@@ -514,7 +516,7 @@ __global__ void __launch_bounds__(AGENT_THREADS, QUEUE ? AGENT_QUEUE_BLOCKS : AG
       nxt = agent_load(st, ni, ni < nblk.end, st.sims[nblk.sim].use_waning != 0);
     }
     agent_block_step<QUEUE>(st, blk, cur, t, do_prev, do_day, full_imm, steady, vq, qn, s_ln_tab, s_ln_inv, s_exp_tab,
-                            nab_fx, sus_fx, symp_fx, acc_prev, acc_day);
+                            s_vl, nab_fx, sus_fx, symp_fx, acc_prev, acc_day);
     if (QUEUE) {
       const bool last = !more || nblk.sim != sim;  // of this sim: the queue is emptied
       __syncwarp();
@@ -532,6 +534,9 @@ __global__ void __launch_bounds__(AGENT_THREADS, QUEUE ? AGENT_QUEUE_BLOCKS : AG
     if (nblk.sim != sim) {
       agent_flush(st, sim, t, do_prev, do_day, sc, nab_fx, sus_fx, symp_fx, acc_prev, acc_day, true);
       sim = nblk.sim;
+      if (threadIdx.x < 2)
+        s_vl[threadIdx.x] = viral_load_of(threadIdx.x == 1, st.sims[sim].frac_time, st.sims[sim].load_ratio);
+      __syncthreads();
     }
     blk = nblk;
     cur = nxt;

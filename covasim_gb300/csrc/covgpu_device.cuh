@@ -265,16 +265,22 @@ __device__ __forceinline__ int64_t roles_words(const covgpu_state& st) { return 
 __device__ __forceinline__ float* dur_row(const covgpu_state& st, int d) { return st.durs + (int64_t)d * st.n; }
 
 // utils.py:39-79 for one agent, float32 as numba types it (the int32 t and the
-// float32 arrays meet in a float32 ufunc loop).
-__device__ __forceinline__ float viral_load_one(int t, float ts, float tr, float td, float frac_time,
-                                                float load_ratio, float high_cap) {
+// float32 arrays meet in a float32 ufunc loop): whether day t is in the early, high
+// part of its infection, and the load of each part (the same for every agent)
+__device__ __forceinline__ bool viral_load_early(int t, float ts, float tr, float td, float frac_time, float high_cap) {
   const float stop = isnan(td) ? tr : td;
   const float total = __fsub_rn(stop, ts);
   const float trans_day = __fmul_rn(frac_time, total);
   const float trans_point = (trans_day > high_cap) ? __fdiv_rn(high_cap, total) : frac_time;
-  const bool early = __fdiv_rn(__fsub_rn((float)t, ts), total) < trans_point;
+  return __fdiv_rn(__fsub_rn((float)t, ts), total) < trans_point;
+}
+__device__ __forceinline__ float viral_load_of(bool early, float frac_time, float load_ratio) {
   const float den = __fadd_rn(1.0f, __fmul_rn(frac_time, __fsub_rn(load_ratio, 1.0f)));
   return __fdiv_rn(early ? load_ratio : 1.0f, den);
+}
+__device__ __forceinline__ float viral_load_one(int t, float ts, float tr, float td, float frac_time,
+                                                float load_ratio, float high_cap) {
+  return viral_load_of(viral_load_early(t, ts, tr, td, frac_time, high_cap), frac_time, load_ratio);
 }
 
 

@@ -266,19 +266,18 @@ __device__ __forceinline__ double exp2_ff(ff x) { return exp2_ff(x, COVGPU_EXP_T
 // calc_VE (immunity.py:216-247) for eff = nab * imm with ln(imm) given:
 // exp(alpha) * eff^beta / (1 + exp(alpha) * eff^beta) = logistic(z),
 // z = alpha + beta * (ln nab + ln imm); rounded once to float32.
+// Without branches, so that an agent's axes run interleaved.
 __device__ __forceinline__ float ve_ff(ff ln_eff, ff alpha, ff beta, const float (*etab)[2]) {
   const ff z = ff_add(alpha, ff_mul(beta, ln_eff));
   const bool pos = z.hi >= 0.0f;
   const ff y = pos ? ff{-z.hi, -z.lo} : z;
-  if (y.hi < -87.0f) return pos ? 1.0f : 0.0f;  // |z| > 87: 1 - 1e-38 rounds to 1; e^-87 flushed to 0
-  const ff x = ff_exp_neg(y, etab);
+  const bool far = y.hi < -87.0f;  // |z| > 87: 1 - 1e-38 rounds to 1; e^-87 flushed to 0
+  const ff x = ff_exp_neg(far ? ff{-87.0f, 0.0f} : y, etab);
   const ff den = fast_two_sum(1.0f, x.hi);
   const ff q = ff_div(x, ff{den.hi, __fadd_rn(den.lo, x.lo)});
-  if (pos) {
-    const ff om = two_sum(1.0f, -q.hi);
-    return __fadd_rn(om.hi, __fsub_rn(om.lo, q.lo));
-  }
-  return __fadd_rn(q.hi, q.lo);
+  const ff om = two_sum(1.0f, -q.hi);
+  const float up = __fadd_rn(om.hi, __fsub_rn(om.lo, q.lo)), low = __fadd_rn(q.hi, q.lo);
+  return far ? (pos ? 1.0f : 0.0f) : (pos ? up : low);
 }
 
 // update_nab (immunity.py:205-213): nab + kin * peak, rounded once to float32,
