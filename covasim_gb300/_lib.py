@@ -184,8 +184,7 @@ def lib():
         L.covgpu_infections_scratch_bytes.restype = i64
         L.covgpu_infections.argtypes = [f32, vp, vp, vp, i64, vp, vp, i64, vp, u64, i32, i32, i32, vp, vp, i64, vp,
                                         vp, vp, i64, vp]
-        L.covgpu_infections_find.argtypes = [f32, vp, vp, vp, i64, vp, vp, i64, vp, u64, i32, i32, i32, vp, vp, vp,
-                                             i64, vp]
+        L.covgpu_infections_find.argtypes = [f32, vp, vp, vp, i64, vp, vp, i64, vp, u64, i32, i32, i32, vp, vp, i64, vp]
         L.covgpu_infections_find.restype = C.c_int
         L.covgpu_infections_emit.argtypes = [vp, vp, i64, vp, i64, vp, vp, vp]
         L.covgpu_infections_emit.restype = C.c_int

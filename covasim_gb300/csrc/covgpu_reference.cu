@@ -486,17 +486,18 @@ int covgpu_infections(float beta, const int32_t* p1, const int32_t* p2, const fl
 int covgpu_infections_find(float beta, const int32_t* p1, const int32_t* p2, const float* layer_betas, int64_t n_edges,
                            const float* rel_trans, const float* rel_sus, int64_t n_agents, const double* uniforms,
                            uint64_t seed, int32_t day, int32_t variant, int32_t layer, int64_t* out_count,
-                           int32_t* status, void* scratch, int64_t scratch_bytes, void* stream) {
+                           void* scratch, int64_t scratch_bytes, void* stream) {
   if (n_edges < 1 || n_edges > FIND_MAX_EDGES || n_agents < 0 || !out_count || !scratch || !p1 || !p2 ||
       !layer_betas || !rel_trans || !rel_sus || variant < 0 || variant >= COVGPU_MAX_VARIANTS || layer < 0 ||
       layer >= COVGPU_MAX_LAYERS || scratch_bytes < find_bytes(n_edges))
     return COVGPU_BADARG;
   InfArgs a;
   a.beta = beta; a.p1 = p1; a.p2 = p2; a.lb = layer_betas; a.E = n_edges; a.rt = rel_trans; a.rs = rel_sus;
-  a.n_agents = n_agents; a.status = status; a.uni = uniforms;
+  a.n_agents = n_agents; a.status = reinterpret_cast<int32_t*>(out_count + 1); a.uni = uniforms;
   a.k0 = (uint32_t)seed; a.k1 = (uint32_t)(seed >> 32); a.day = day; a.variant = variant; a.layer = layer;
   int blocks = 0;
   const FindArgs f = find_args(a, scratch, out_count, blocks);
+  if (cudaMemsetAsync(out_count, 0, 2 * sizeof(int64_t), S(stream)) != cudaSuccess) return COVGPU_CUDA_ERROR;
   k_inf_find<<<blocks, FIND_THREADS, 0, S(stream)>>>(f);
   return launch_status();
 }

@@ -80,12 +80,12 @@ def _infections_call(beta, p1, p2, layer_betas, rel_trans, rel_sus, uniforms, se
     if E == 0:
         return torch.empty(0, dtype=_I32, device=dev), torch.empty(0, dtype=_I32, device=dev)
     n_agents = min(rel_trans.numel(), rel_sus.numel())
-    count = torch.zeros(2, dtype=torch.int64, device=dev)  # transmissions, status
+    count = torch.empty(2, dtype=torch.int64, device=dev)  # transmissions, status
     nbytes = int(L.lib().covgpu_infections_scratch_bytes(E))
     scratch = torch.empty(nbytes, dtype=_U8, device=dev)
     L.call('covgpu_infections_find', float(beta), _ptr(p1), _ptr(p2), _ptr(layer_betas), E, _ptr(rel_trans),
            _ptr(rel_sus), n_agents, _ptr(uniforms), int(seed) & 0xFFFFFFFFFFFFFFFF, int(day), int(variant), int(layer),
-           count.data_ptr(), count.data_ptr() + 8, scratch.data_ptr(), nbytes, _raw_stream(count))
+           count.data_ptr(), scratch.data_ptr(), nbytes, _raw_stream(count))
     n, status = count.tolist()
     if status & L.BADARG:
         raise IndexError('compute_infections: an edge index is outside the agent arrays')

@@ -435,16 +435,16 @@ int covgpu_infections(float beta, const int32_t* p1, const int32_t* p2, const fl
                       int32_t* status, void* scratch, int64_t scratch_bytes, void* stream);
 
 /* compute_infections in two calls, for callers that allocate outputs of the
- * exact size: _find evaluates every edge (1 <= n_edges <= 2^36), adds the
- * number of transmissions to *out_count and ORs COVGPU_BADARG into *status
- * for a bad edge (device, cleared by the caller; status may be NULL); _emit
+ * exact size: _find evaluates every edge (1 <= n_edges <= 2^36) and sets
+ * out_count[0] to the number of transmissions and out_count[1] to 0 or, for a
+ * bad edge, COVGPU_BADARG (device); _emit
  * then writes the first `count` transmissions from the same scratch, which
  * must not change in between. scratch: covgpu_infections_scratch_bytes(n_edges)
  * bytes. */
 int covgpu_infections_find(float beta, const int32_t* p1, const int32_t* p2, const float* layer_betas,
                            int64_t n_edges, const float* rel_trans, const float* rel_sus, int64_t n_agents,
                            const double* uniforms, uint64_t seed, int32_t day, int32_t variant, int32_t layer,
-                           int64_t* out_count, int32_t* status, void* scratch, int64_t scratch_bytes, void* stream);
+                           int64_t* out_count, void* scratch, int64_t scratch_bytes, void* stream);
 int covgpu_infections_emit(const int32_t* p1, const int32_t* p2, int64_t n_edges, const void* scratch,
                            int64_t count, int32_t* out_src, int32_t* out_tgt, void* stream);
 
