@@ -334,6 +334,7 @@ constexpr int PASS_BLOCKS = 8;
 template <bool MARK>
 __global__ void __launch_bounds__(AGENT_THREADS, PASS_BLOCKS) k_test_pass(covgpu_state st, int t) {
   pdl_wait();
+  pdl_trigger();  // one wave, all resident: the next kernel's set-up overlaps this pass
   if (held(st, t)) return;
   int64_t b, b_end;
   if (!agent_range(st, b, b_end)) return;
@@ -354,7 +355,6 @@ __global__ void __launch_bounds__(AGENT_THREADS, PASS_BLOCKS) k_test_pass(covgpu
     }
     test_block<MARK>(st, t, blk, f, dd, tested_acc);
   }
-  pdl_trigger();
   test_flush(st, t, sim, tested_acc);
 }
 
@@ -545,6 +545,7 @@ __device__ __forceinline__ void post_flush(const covgpu_state& st, int t, int si
 
 __global__ void __launch_bounds__(AGENT_THREADS, PASS_BLOCKS) k_post_pass(covgpu_state st, int t) {
   pdl_wait();
+  pdl_trigger();  // one wave, all resident: the next kernel's set-up overlaps this pass
   if (held(st, t)) return;
   int64_t b, b_end;
   if (!agent_range(st, b, b_end)) return;
@@ -573,7 +574,6 @@ __global__ void __launch_bounds__(AGENT_THREADS, PASS_BLOCKS) k_post_pass(covgpu
     }
     post_block(st, t, blk, in, acc_diag, acc_quar, acc_iso);
   }
-  pdl_trigger();
   post_flush(st, t, sim, acc_diag, acc_quar, acc_iso);
 }
 
