@@ -72,57 +72,88 @@ __device__ __forceinline__ uint64_t swab_threshold(const covgpu_state& st, const
 }
 
 // contact_tracing.identify_contacts, the find_contacts half (utils.py:131-147), for
-// the traced agents of one warp's 32 (bit r of `traced`: agent i0 + r): each marks
-// the other endpoint of its edges in the layers' bitmaps. A traced agent's layers
-// are spread over four groups of eight lanes, whose lanes share its edges: as p1
-// and p2 through a stored layer's index, and the partners of its two lists (the
-// draws the edge pass makes for that agent as a source) in a redrawn layer. The
-// chain of dependent loads (row, edge, endpoint) is paid about once per traced
-// agent instead of once per edge. In a 300,000-agent sim (a median day): the test
-// pass with the marks 17.0 us, against 7.8 us without them, 21.1 us for a thread of
-// its own per traced agent and 12.4 us for the redrawn layer's lists, three
-// launches.
+// one layer of one traced agent: the other endpoint of each of its edges is marked in
+// the layer's bitmap by a group of MARK_LANES lanes (sub: the lane within it), as p1
+// and p2 through a stored layer's index, and the partners of its two lists (the draws
+// the edge pass makes for that agent as a source) in a redrawn layer.
 constexpr int MARK_LANES = 8;
-__device__ __noinline__ void mark_contacts(const covgpu_state& st, const covgpu_sim_params& sp, int64_t i0, uint32_t traced, int t) {
-  const covgpu_testing& T = sp.testing;
-  const int lane = threadIdx.x & 31, sub = lane & (MARK_LANES - 1);
-  const int64_t words = (st.n + 31) >> 5;
+__device__ __noinline__ void mark_layer(const covgpu_state& st, const covgpu_sim_params& sp, uint32_t a, int l, int sub,
+                                        int t) {
+  const int seg = l < sp.n_layers ? sp.seg_of_layer[l] : -1;
+  if (seg < 0 || sp.testing.thr_trace[l] == 0) return;
+  const covgpu_layer& L = st.segments[seg];
   const int32_t off = (int32_t)sp.agent_off;
-  const uint32_t n_local = (uint32_t)sp.n_agents;
-  for (; traced; traced &= traced - 1) {
-    const uint32_t a = (uint32_t)(i0 + (__ffs(traced) - 1) - off);
-    for (int l = lane / MARK_LANES; l < sp.n_layers; l += 32 / MARK_LANES) {
-      const int seg = sp.seg_of_layer[l];
-      if (seg < 0 || T.thr_trace[l] == 0) continue;
-      const covgpu_layer& L = st.segments[seg];
-      uint32_t* contact = st.contact_bits + (int64_t)l * words;
-      if (L.dynamic) {
-        int k[2];
-        dyn_counts(L.dyn_cdf, L.dyn_k, a, (uint32_t)t, (uint32_t)l, sp.key0, sp.key1, k[0], k[1]);
-        const uint32_t thr = bounded_thr(n_local);
-        const int nb0 = (k[0] + 3) >> 2, nb = nb0 + ((k[1] + 3) >> 2);  // four-entry blocks of both lists
-        for (int b = sub; b < nb; b += MARK_LANES) {
-          const int d = b >= nb0 ? 1 : 0, j0 = 4 * (d ? b - nb0 : b);
-          const uint4 pw = dyn_partner_block(a, d, j0, (uint32_t)t, (uint32_t)l, sp.key0, sp.key1);
-          for (int j = j0; j < j0 + 4 && j < k[d]; ++j) {
-            const int32_t g = off + (int32_t)dyn_partner(word_of(pw, j & 3), n_local, thr, a, d, j, (uint32_t)t,
-                                                         (uint32_t)l, sp.key0, sp.key1);
-            atomicOr(contact + (g >> 5), 1u << (g & 31));
-          }
-        }
-      } else if (L.rp1) {
-        const uint32_t b1 = L.rp1[a], e1 = L.rp1[a + 1], b2 = L.rp2[a], e2 = L.rp2[a + 1];
-        for (uint32_t k = b1 + sub; k < e1; k += MARK_LANES) {
-          const int32_t g = L.p2[k];
-          atomicOr(contact + (g >> 5), 1u << (g & 31));
-        }
-        for (uint32_t k = b2 + sub; k < e2; k += MARK_LANES) {
-          const int32_t g = L.rev1 ? L.rev1[k] : L.p1[L.perm2[k]];
-          atomicOr(contact + (g >> 5), 1u << (g & 31));
-        }
+  uint32_t* contact = st.contact_bits + (int64_t)l * ((st.n + 31) >> 5);
+  if (L.dynamic) {
+    const uint32_t n_local = (uint32_t)sp.n_agents, thr = bounded_thr(n_local);
+    int k[2];
+    dyn_counts(L.dyn_cdf, L.dyn_k, a, (uint32_t)t, (uint32_t)l, sp.key0, sp.key1, k[0], k[1]);
+    const int nb0 = (k[0] + 3) >> 2, nb = nb0 + ((k[1] + 3) >> 2);  // four-entry blocks of both lists
+    for (int b = sub; b < nb; b += MARK_LANES) {
+      const int d = b >= nb0 ? 1 : 0, j0 = 4 * (d ? b - nb0 : b);
+      const uint4 pw = dyn_partner_block(a, d, j0, (uint32_t)t, (uint32_t)l, sp.key0, sp.key1);
+      for (int j = j0; j < j0 + 4 && j < k[d]; ++j) {
+        const int32_t g = off + (int32_t)dyn_partner(word_of(pw, j & 3), n_local, thr, a, d, j, (uint32_t)t,
+                                                     (uint32_t)l, sp.key0, sp.key1);
+        atomicOr(contact + (g >> 5), 1u << (g & 31));
       }
     }
+  } else if (L.rp1) {
+    const uint32_t b1 = L.rp1[a], e1 = L.rp1[a + 1], b2 = L.rp2[a], e2 = L.rp2[a + 1];
+    for (uint32_t k = b1 + sub; k < e1; k += MARK_LANES) {
+      const int32_t g = L.p2[k];
+      atomicOr(contact + (g >> 5), 1u << (g & 31));
+    }
+    for (uint32_t k = b2 + sub; k < e2; k += MARK_LANES) {
+      const int32_t g = L.rev1 ? L.rev1[k] : L.p1[L.perm2[k]];
+      atomicOr(contact + (g >> 5), 1u << (g & 31));
+    }
+  }
+}
+
+// The traced agents of one thread block's agent-block range, in shared memory: once
+// the range is done (mark_block), the (layer, agent) pairs are shared by the block's
+// groups of lanes, a warp's groups on the same layer where there are enough agents,
+// so that the chains of dependent loads (row, edge, endpoint, or the lists' draws)
+// run side by side instead of one after another in the warp that found the agent
+// (10M agents with testing: 91.2 -> 89.7 ms a run). A median day of 300,000 agents: the
+// test pass with the marks 14.3 us, against 7.8 us without them, 21.1 us for a thread
+// of its own per traced agent and 12.4 us for the redrawn layer's lists, three
+// launches.
+constexpr int MARK_CAP = 512;
+struct MarkList {
+  uint32_t agent[MARK_CAP];
+  unsigned n;
+};
+// the traced agents of one warp's 32 (bit r: agent i0 + r); those past the list's end
+// are marked here, by the whole warp
+__device__ __forceinline__ void mark_push(const covgpu_state& st, const covgpu_sim_params& sp, int64_t i0,
+                                          uint32_t traced, int t, MarkList& list) {
+  const int lane = threadIdx.x & 31;
+  unsigned pos = 0;
+  if (lane == 0) pos = atomicAdd(&list.n, (unsigned)__popc(traced));
+  pos = __shfl_sync(0xffffffffu, pos, 0) + __popc(traced & ((1u << lane) - 1u));
+  const bool mine = (traced >> lane) & 1u;
+  if (mine && pos < MARK_CAP) list.agent[pos] = (uint32_t)(i0 + lane);
+  for (unsigned over = __ballot_sync(0xffffffffu, mine && pos >= MARK_CAP); over; over &= over - 1) {
+    const uint32_t a = (uint32_t)(i0 + (__ffs(over) - 1) - sp.agent_off);
+    for (int l = lane / MARK_LANES; l < sp.n_layers; l += 32 / MARK_LANES)
+      mark_layer(st, sp, a, l, lane & (MARK_LANES - 1), t);
     __syncwarp();
+  }
+}
+__device__ __forceinline__ void mark_block(const covgpu_state& st, int t, const MarkList& list) {
+  __syncthreads();
+  const unsigned n = min(list.n, (unsigned)MARK_CAP);
+  for (unsigned j = threadIdx.x / MARK_LANES; j < n * (unsigned)st.n_contact_layers; j += AGENT_THREADS / MARK_LANES) {
+    const uint32_t i = list.agent[j % n];
+    int lo = 0, hi = st.n_sims - 1;  // the agent's sim
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (st.sims[mid].agent_off <= (int64_t)i) lo = mid; else hi = mid - 1;
+    }
+    const covgpu_sim_params& sp = st.sims[lo];
+    mark_layer(st, sp, (uint32_t)((int64_t)i - sp.agent_off), (int)(j / n), threadIdx.x & (MARK_LANES - 1), t);
   }
 }
 
@@ -130,11 +161,10 @@ __device__ __noinline__ void mark_contacts(const covgpu_state& st, const covgpu_
 // then the agents contact_tracing.select_cases picks (interventions.py:1066-1072).
 // One agent block of the test pass (thread k on agent begin + k, its flags f and
 // diagnosis date dd already loaded); the tested are counted into the thread's
-// accumulator. MARK: the traced agents' contacts are marked here, else the traced
-// go to their bitmap.
+// accumulator. MARK: the traced go to the block's list, else to their bitmap.
 template <bool MARK>
 __device__ __forceinline__ void test_block(const covgpu_state& st, int t, const covgpu_agent_block& blk, uint32_t f,
-                                           float dd, unsigned& tested_acc) {
+                                           float dd, unsigned& tested_acc, MarkList& list) {
   const covgpu_sim_params& sp = st.sims[blk.sim];
   const covgpu_testing& T = sp.testing;
   const bool test_on = day_active(t, T.test_start, T.test_end);
@@ -193,7 +223,7 @@ __device__ __forceinline__ void test_block(const covgpu_state& st, int t, const 
   tested_acc += tested;
   const uint32_t tm = __ballot_sync(0xffffffffu, trace);
   if (MARK) {
-    if (tm) mark_contacts(st, sp, blk.begin + warp * 32, tm, t);
+    if (tm) mark_push(st, sp, blk.begin + warp * 32, tm, t, list);
     return;
   }
   if (trace_on && lane == 0 && blk.begin + warp * 32 < blk.end) st.trace_bits[(blk.begin + warp * 32) >> 5] = tm;
@@ -338,6 +368,9 @@ __global__ void __launch_bounds__(AGENT_THREADS, PASS_BLOCKS) k_test_pass(covgpu
   if (held(st, t)) return;
   int64_t b, b_end;
   if (!agent_range(st, b, b_end)) return;
+  __shared__ MarkList s_list;
+  if (threadIdx.x == 0) s_list.n = 0;
+  __syncthreads();
   int sim = st.agent_blocks[b].sim;
   unsigned tested_acc = 0;
   for (; b < b_end; ++b) {
@@ -353,9 +386,10 @@ __global__ void __launch_bounds__(AGENT_THREADS, PASS_BLOCKS) k_test_pass(covgpu
       test_flush(st, t, sim, tested_acc);
       sim = blk.sim;
     }
-    test_block<MARK>(st, t, blk, f, dd, tested_acc);
+    test_block<MARK>(st, t, blk, f, dd, tested_acc, s_list);
   }
   test_flush(st, t, sim, tested_acc);
+  if (MARK) mark_block(st, t, s_list);
 }
 
 // The marking on its own, from the test pass's bitmap of the traced (after the
@@ -364,6 +398,9 @@ __global__ void __launch_bounds__(AGENT_THREADS) k_trace_marks(covgpu_state st, 
   if (held(st, t)) return;
   int64_t b, b_end;
   if (!agent_range(st, b, b_end)) return;
+  __shared__ MarkList s_list;
+  if (threadIdx.x == 0) s_list.n = 0;
+  __syncthreads();
   const int warp = threadIdx.x >> 5;
   for (; b < b_end; ++b) {
     const covgpu_agent_block blk = st.agent_blocks[b];
@@ -373,8 +410,9 @@ __global__ void __launch_bounds__(AGENT_THREADS) k_trace_marks(covgpu_state st, 
         st.trace_count[blk.sim] == 0)
       continue;
     const uint32_t tm = st.trace_bits[i0 >> 5];
-    if (tm) mark_contacts(st, sp, i0, tm, t);
+    if (tm) mark_push(st, sp, i0, tm, t, s_list);
   }
+  mark_block(st, t, s_list);
 }
 
 __device__ __forceinline__ uint32_t bit_of(const uint32_t* __restrict__ bits, int32_t a) {
@@ -383,7 +421,7 @@ __device__ __forceinline__ uint32_t bit_of(const uint32_t* __restrict__ bits, in
 
 // contact_tracing.identify_contacts, the find_contacts half (utils.py:131-147):
 // every edge of a stored layer without an index with a traced endpoint marks the
-// other endpoint in its layer's bitmap (the others: mark_contacts)
+// other endpoint in its layer's bitmap (the others: mark_layer)
 template <int ROUNDS>
 __global__ void __launch_bounds__(EDGE_THREADS) k_trace_scan(covgpu_state st, int t) {
   if (held(st, t)) return;
@@ -402,7 +440,7 @@ __global__ void __launch_bounds__(EDGE_THREADS) k_trace_scan(covgpu_state st, in
   const covgpu_sim_params& sp = st.sims[L->sim];
   const covgpu_testing& T = sp.testing;
   if (!day_active(t, T.trace_start, T.trace_end) || T.thr_trace[L->layer] == 0 || st.trace_count[L->sim] == 0) return;
-  if (L->rp1) return;  // indexed: mark_contacts visits the traced agents' edges
+  if (L->rp1) return;  // indexed: mark_layer visits the traced agents' edges
   const int64_t words = (st.n + 31) >> 5;
   uint32_t* contact = st.contact_bits + (int64_t)L->layer * words;
   const int64_t e0 = ((int64_t)blockIdx.x - L->tile_begin) * TILE;
