@@ -1135,18 +1135,20 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_edge_pass_res(covgpu_state s
 // ============================================================ redrawn layers
 //
 // Transmission over the dynamic layers (base.py:1849-1876 redrawn daily, then
-// utils.py:93-128): one warp per agent block of one sim, or two (source_split), on its
+// utils.py:93-128): one warp or more per agent block of one sim (source_split), on its
 // source-bitmap words. The words' sources are handed to the lanes 32 at a time; for each
 // dynamic layer of the sim every lane draws its source's two list lengths
 // (covgpu_device.cuh, "redrawn layers, per agent"), and the lists' four-entry
 // blocks of all 32 sources are then spread over the lanes (a prefix count and a
 // search for each block's source), so that the Philox blocks of a warp with few
 // sources still run on full lanes. Entries are thinned (covgpu_device.cuh
-// "Thinning"): only the potential transmissions, about pmax of them, have their
-// partner drawn, and those whose partner is a target are queued; the queue
-// drains through edge_try as the stored layers' does. The work follows the
-// day's sources, not the layer's edges: a quiet day costs a read of the source
-// bitmap.
+// "Thinning"): only the potential transmissions, about pmax of them, are queued, and
+// on draining have their partner drawn and, where it is a target, go through edge_try
+// as the stored layers' candidates do. (Drawn where they were found, the partners of
+// the few lanes with one cost the whole warp a Philox block each round: 1M agents
+// 15.45 -> 15.06 ms a run.) The likelihood, which takes every entry, draws all
+// partners first and queues those that are targets. The work follows the day's
+// sources, not the layer's edges: a quiet day costs a read of the source bitmap.
 constexpr int DYN_WARPS = 8;  // warps per thread block
 // Warps per agent block of the per-source passes (split: each warp takes 8 / split
 // of the agent block's eight source-bitmap words): one from SPLIT_TARGET agent
@@ -1221,6 +1223,32 @@ __device__ __forceinline__ void dyn_drain(const covgpu_state& st, const SegCtx& 
   emit(st, hit, hit ? event_key(t, v, c.layer, (int)(m & 1u), (int64_t)e) : 0ull, g, s);
 }
 
+// The potential transmissions [base, base + 32) of the queue (those below qn), one per
+// lane: the entry's partner (only a potential transmission needs one), and if it is a
+// target the edge's own draw, then the warp-aggregated event append (m = j << 1 | d)
+__device__ __forceinline__ void dyn_potential_drain(const covgpu_state& st, const SegCtx& c, int t, int32_t off,
+                                                    uint32_t n_local, uint32_t thr, const EdgeQueue& q, int base,
+                                                    int qn, LikAcc& acc) {
+  const int i = base + (threadIdx.x & 31);
+  bool hit = false;
+  uint32_t v = 0, m = 0;
+  int32_t s = 0, g = 0;
+  uint64_t e = 0;
+  if (i < qn) {
+    s = q.s[i];
+    m = q.m[i];
+    const uint32_t a = (uint32_t)(s - off), day = (uint32_t)t, layer = (uint32_t)c.layer;
+    const int j = (int)(m >> 1), d = (int)(m & 1u);
+    const uint4 pw = dyn_partner_block(a, d, j, day, layer, c.key0, c.key1);
+    g = off + (int32_t)dyn_partner(word_of(pw, j & 3), n_local, thr, a, d, j, day, layer, c.key0, c.key1);
+    if (tgt_bit(st, g)) {
+      e = dyn_edge_id(a, (uint32_t)j, day, layer);
+      hit = edge_try<false, false, true>(st, c, t, (int64_t)e, d, s, g, v, acc);
+    }
+  }
+  emit(st, hit, hit ? event_key(t, v, c.layer, (int)(m & 1u), (int64_t)e) : 0ull, g, s);
+}
+
 // The redrawn layers of the day's sources for one block's worth (vblock) of
 // agent blocks: split warps per agent block, each on AB_WORDS / split source-bitmap words.
 template <bool LIK>
@@ -1284,33 +1312,53 @@ __device__ __forceinline__ void dyn_body(const covgpu_state& st, int t, int64_t 
         const int ok0 = __shfl_sync(0xffffffffu, k0, owner), ok1 = __shfl_sync(0xffffffffu, k1, owner);
         const uint32_t onb0 = __shfl_sync(0xffffffffu, nb0, owner);
         const uint32_t obeg = __shfl_sync(0xffffffffu, pre - nb, owner);
-        uint32_t pm = 0u, tb = 0u;
-        int d = 0, je = 0;
-        int32_t g[4] = {0, 0, 0, 0};
+        uint32_t pm = 0u;
+        int d = 0, je = 0, kd = 0;
         if (j < total) {
           const uint32_t r = j - obeg;
           d = r >= onb0 ? 1 : 0;
           je = 4 * (int)(d ? r - onb0 : r);
-          const int kd = d ? ok1 : ok0;
-          const uint32_t oa = (uint32_t)(os - off);
+          kd = d ? ok1 : ok0;
           if (om >= 0) {  // potential transmissions among entries je .. je + 3
-            const uint4 hw = dyn_hit_block(oa, d, je, day, (uint32_t)l, c.key0, c.key1);
+            const uint4 hw = dyn_hit_block((uint32_t)(os - off), d, je, day, (uint32_t)l, c.key0, c.key1);
 #pragma unroll
             for (int r4 = 0; r4 < 4; ++r4)
               if (je + r4 < kd && thin_potential(word_of(hw, r4), om)) pm |= 1u << r4;
           }
-          // partners: of the potential entries (all entries for the likelihood)
-          const uint32_t want = LIK ? (0xFu >> max(0, 4 - (kd - je))) : pm;
-          if (want) {
-            const uint4 pw = dyn_partner_block(oa, d, je, day, (uint32_t)l, c.key0, c.key1);
-#pragma unroll
-            for (int r4 = 0; r4 < 4; ++r4)
-              if ((want >> r4) & 1u) {
-                g[r4] = off + (int32_t)dyn_partner(word_of(pw, r4), n_local, thr, oa, d, je + r4, day, (uint32_t)l,
-                                                   c.key0, c.key1);
-                tb |= tgt_bit(st, g[r4]) << r4;
-              }
+        }
+        if (!LIK) {
+          // a few of the warp's entries are potential transmissions: queued (usually one
+          // round, each lane its lowest), and partner, target and draw on full warps
+          for (unsigned any = __ballot_sync(0xffffffffu, pm != 0u); any; any = __ballot_sync(0xffffffffu, pm != 0u)) {
+            if (pm) {
+              const int pos = qn + __popc(any & ((1u << lane) - 1u));
+              q.s[pos] = os;
+              q.m[pos] = (uint16_t)((uint32_t)(je + __ffs(pm) - 1) << 1 | (uint32_t)d);
+              pm &= pm - 1u;
+            }
+            qn += __popc(any);
           }
+          __syncwarp();
+          while (qn >= 32) {  // full warps from the top of the queue
+            qn -= 32;
+            dyn_potential_drain(st, c, t, off, n_local, thr, q, qn, qn + 32, acc);
+          }
+          __syncwarp();
+          continue;
+        }
+        // the likelihood takes every entry: all partners are drawn
+        uint32_t tb = 0u;
+        int32_t g[4] = {0, 0, 0, 0};
+        if (j < total) {
+          const uint32_t oa = (uint32_t)(os - off);
+          const uint4 pw = dyn_partner_block(oa, d, je, day, (uint32_t)l, c.key0, c.key1);
+#pragma unroll
+          for (int r4 = 0; r4 < 4; ++r4)
+            if (je + r4 < kd) {
+              g[r4] = off + (int32_t)dyn_partner(word_of(pw, r4), n_local, thr, oa, d, je + r4, day, (uint32_t)l,
+                                                 c.key0, c.key1);
+              tb |= tgt_bit(st, g[r4]) << r4;
+            }
         }
         if (!__any_sync(0xffffffffu, tb != 0u)) continue;
 #pragma unroll
@@ -1325,7 +1373,10 @@ __device__ __forceinline__ void dyn_body(const covgpu_state& st, int t, int64_t 
         __syncwarp();
       }
     }
-    if (qn > 0) dyn_drain<LIK>(st, c, t, sp.agent_off, q, 0, qn, acc);
+    if (qn > 0) {
+      if (LIK) dyn_drain<LIK>(st, c, t, sp.agent_off, q, 0, qn, acc);
+      else dyn_potential_drain(st, c, t, off, n_local, thr, q, 0, qn, acc);
+    }
     if (LIK) lik_flush_warp(st, t, blk.sim, l, acc);
     __syncwarp();  // the queue is read before the next layer fills it
   }
