@@ -270,16 +270,21 @@ def ili_agents(seed, t, n, n_ili):
 # * no redrawn layer: walked every day, and the tile pass is not launched (96
 #   random-population sims, 115M edges, 120 days: 83.5 ms a batched run, 106.3 ms
 #   walking below 1/64 infectious and 107.2 ms below 1/8, two launches a day);
-# * a redrawn layer, below SRC_WALK_ALL_AGENTS agents: walked every day, one launch
-#   with the redrawn layer's pass instead of a fork and join of two (300,000 agents,
-#   testing: 6.97 ms a run, 7.29 below 1/128); above, the stream beside the redrawn
-#   layer's pass is faster on the busy days (1M agents: 15.9 ms below 1/16, 17.3
-#   every day, 16.0 below 1/128; 10M: 105.4, 105.2, 111.3);
+# * a redrawn layer and testing, below SRC_WALK_ALL_AGENTS agents: walked every day,
+#   one launch with the redrawn layer's pass instead of a fork and join of two (ms a
+#   120-day run, every day / below 1/16 / below 1/128: 200,000 agents 6.40, 6.76, 6.57;
+#   300,000 6.85, 7.25, 7.15; 600,000 9.32, 9.74, 9.39); above, below 1/16 (10M with
+#   three variants 105.2, 105.4, 111.3);
+# * a redrawn layer without testing: below 1/32, the stream beside the redrawn layer's
+#   pass being faster on the busy days (every day / 1/16 / 1/32 / 1/128: 30,000 agents
+#   3.51, 3.43, 3.41, 3.38; 300,000 5.75, 5.59, 5.55, 5.55; 1M, 150 days, 14.75, 13.25,
+#   13.12, 13.27; 3M, 100 days, 23.8, 21.4, 21.5, 22.0);
 # * with the likelihood, whose walk takes the layers one after another, SRC_WALK
 #   (100,000 agents: 7.96 ms, 8.44 every day).
 SRC_WALK = 128
-SRC_WALK_REDRAWN = 16
-SRC_WALK_ALL_AGENTS = 500_000
+SRC_WALK_TESTING = 16
+SRC_WALK_REDRAWN = 32
+SRC_WALK_ALL_AGENTS = 600_000
 SRC_WALK_BIG = 64
 SRC_WALK_MIN_EDGES = 50_000_000
 
@@ -772,7 +777,9 @@ class BatchState:
             if not any(rec.dynamic for rec in self.segments):
                 k = -1
             elif not self.lik_active:
-                k = -1 if self.n < SRC_WALK_ALL_AGENTS else SRC_WALK_REDRAWN
+                k = SRC_WALK_REDRAWN
+                if self.has_testing:
+                    k = -1 if self.n < SRC_WALK_ALL_AGENTS else SRC_WALK_TESTING
         return L.WALK_ALL if indexed and k == -1 else k
 
     def set_src_walk(self, k):

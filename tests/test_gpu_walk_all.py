@@ -26,6 +26,8 @@ def test_walk_every_day_equals_streamed(pop_type, n, dyn, trace):
         sim = cv.Sim(pars)
         sim.initialize()
         if mode is None:
+            assert sim.state.cstate.src_walk == (L.WALK_ALL if trace else 32)
+            sim.state.set_src_walk(-1)
             assert sim.state.cstate.src_walk == L.WALK_ALL
         else:
             sim.state.set_src_walk(mode)
