@@ -263,13 +263,20 @@ def ili_agents(seed, t, n, n_ili):
 
 # When the stored layers are walked from the day's sources (covgpu_state.src_walk;
 # results are the same either way). BatchState.src_walk is the threshold k of a
-# state with a redrawn layer (SRC_WALK) or of one whose stored edges make a day's
-# stream long (SRC_WALK_BIG, from SRC_WALK_MIN_EDGES edges); both build the agent
-# index the walk needs, as tracing does. Until set_src_walk asks for a threshold,
-# _walk_mode refines it from sizes once every stored layer has its index:
-# * no redrawn layer: walked every day, and the tile pass is not launched (96
-#   random-population sims, 115M edges, 120 days: 83.5 ms a batched run, 106.3 ms
-#   walking below 1/64 infectious and 107.2 ms below 1/8, two launches a day);
+# state with a redrawn layer (SRC_WALK), or without one of a state whose stored
+# edges make a day's stream long (SRC_WALK_BIG, from SRC_WALK_MIN_EDGES edges in one
+# sim, SRC_WALK_MIN_EDGES_BATCH in several); both build the agent index the walk
+# needs, as tracing does. Until set_src_walk asks for a threshold, _walk_mode refines
+# it from sizes once every stored layer has its index (ms a run; "every day" also
+# leaves out the tile pass's launch):
+# * one sim without a redrawn layer: below 1/16 (100-120 days, streamed / every day /
+#   1/16: random 700,000 agents, 7M edges, 8.38, -, 8.13; 1M 11.7, -, 10.8; 2M 23.0,
+#   20.9, 17.8; hybrid 1M, 17.8M edges, 15.9, 15.7, 14.0; building the index takes
+#   0.5 ms at 1M); with tracing, which has the index anyway, every day from
+#   SRC_WALK_TRACE_AGENTS (hybrid 20,000 agents 3.45, 3.72, 4.08; 100,000 3.81, 3.79,
+#   4.19; 300,000 5.23, 5.06, 5.46; 1M 10.97, 9.24, 9.69; 4M 18.0, 10.2, 10.3);
+# * several: every day (24 to 96 random sims, streamed / every day / 1/64: 17M edges
+#   16.0, 18.1, 16.9; 30M 24.6, 24.6, 24.6; 43M 33.1, 29.2, 31.7; 115M -, 83.5, 106);
 # * a redrawn layer and testing, below SRC_WALK_ALL_AGENTS agents: walked every day,
 #   one launch with the redrawn layer's pass instead of a fork and join of two (ms a
 #   120-day run, every day / below 1/16 / below 1/128: 200,000 agents 6.40, 6.76, 6.57;
@@ -286,7 +293,10 @@ SRC_WALK_TESTING = 16
 SRC_WALK_REDRAWN = 32
 SRC_WALK_ALL_AGENTS = 600_000
 SRC_WALK_BIG = 64
-SRC_WALK_MIN_EDGES = 50_000_000
+SRC_WALK_MIN_EDGES = 10_000_000
+SRC_WALK_MIN_EDGES_BATCH = 30_000_000
+SRC_WALK_ONE = 16
+SRC_WALK_TRACE_AGENTS = 150_000
 
 
 def parse_edge_tile(choice):
@@ -316,7 +326,8 @@ class BatchState:
             self.src_walk = SRC_WALK
         else:
             stored = sum(len(ly['p1']) for sp in specs for ly in sp.layers)
-            self.src_walk = SRC_WALK_BIG if stored >= SRC_WALK_MIN_EDGES else 0
+            least = SRC_WALK_MIN_EDGES if len(specs) == 1 else SRC_WALK_MIN_EDGES_BATCH
+            self.src_walk = SRC_WALK_BIG if stored >= least else 0
         self._walk_default = True  # until set_src_walk
         self._index_pending = []  # stored segments whose agent index is built on demand
         self._index_tensors = []
@@ -773,13 +784,18 @@ class BatchState:
         default rule (above) until one is asked for."""
         k = int(self.src_walk)
         indexed = all(rec.dynamic or rec.rp1 for rec in self.segments)
-        if self._walk_default and indexed:
-            if not any(rec.dynamic for rec in self.segments):
-                k = -1
-            elif not self.lik_active:
+        if self._walk_default and indexed and not self.lik_active:
+            dynamic = any(rec.dynamic for rec in self.segments)
+            if dynamic and self.has_testing:
+                k = -1 if self.n < SRC_WALK_ALL_AGENTS else SRC_WALK_TESTING
+            elif dynamic:
                 k = SRC_WALK_REDRAWN
-                if self.has_testing:
-                    k = -1 if self.n < SRC_WALK_ALL_AGENTS else SRC_WALK_TESTING
+            elif len(self.specs) > 1:
+                k = -1 if k else 0
+            elif self.has_testing:
+                k = -1 if self.n >= SRC_WALK_TRACE_AGENTS else 0
+            else:
+                k = SRC_WALK_ONE
         return L.WALK_ALL if indexed and k == -1 else k
 
     def set_src_walk(self, k):

@@ -26,7 +26,7 @@ def test_walk_every_day_equals_streamed(pop_type, n, dyn, trace):
         sim = cv.Sim(pars)
         sim.initialize()
         if mode is None:
-            assert sim.state.cstate.src_walk == (L.WALK_ALL if trace else 32)
+            assert sim.state.cstate.src_walk == (32 if dyn else (L.WALK_ALL if n >= 150_000 else 0))
             sim.state.set_src_walk(-1)
             assert sim.state.cstate.src_walk == L.WALK_ALL
         else:
