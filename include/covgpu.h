@@ -230,7 +230,7 @@ typedef struct covgpu_sim_params {
  * distribution: dyn_cdf[k] = floor(2^64 * P(count <= k)) for k < dyn_k - 1
  * and dyn_cdf[dyn_k - 1] = 2^64 - 1, with dyn_k <= COVGPU_DYN_MAX_LIST. */
 #define COVGPU_DYN_MAX_LIST 1024
-#define COVGPU_WALK_ALL (-2)      /* covgpu_state.src_walk */
+#define COVGPU_WALK_ALL (-2147483647 - 1)  /* covgpu_state.src_walk */
 typedef struct covgpu_layer {
   const int32_t* p1;              /* global agent indices, sorted ascending (static) */
   const int32_t* p2;
