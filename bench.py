@@ -51,12 +51,13 @@ RECORDED_CUM_INFECTIONS = {(1_000_000, 180, 1): 1_055_079}
 
 MEASURED_NCU = {
     ('agent_step', 1_000_000): {
-        'dram_bytes': 69_901_568, 'issue_active': 0.602, 'bound': 'issue',
-        'note': 'ncu section capture, day 85 of the 1M-agent run: 69.9 MB of DRAM traffic against 88 MB '
-                'algorithmic; instruction issue 60% busy, 35.0 M warp instructions for 1M agents, so the pass '
+        'dram_bytes': 75_929_088, 'issue_active': 0.625, 'bound': 'issue',
+        'note': 'ncu section capture, day 85 of the 1M-agent run: 75.9 MB of DRAM traffic against 88 MB '
+                'algorithmic; instruction issue 62% busy, 38.9 M warp instructions for 1M agents (with the '
+                'severe efficacy, stored on a sequence\'s last day only), so the pass '
                 'is issue-bound on the float-float efficacies, not HBM-bound'},
     ('edge_stored', 1_000_000): {
-        'dram_bytes': 83_445_760, 'issue_active': 0.533, 'bound': 'latency',
+        'dram_bytes': 83_339_008, 'issue_active': 0.574, 'bound': 'latency',
         'note': 'ncu section capture, day 85 (one-wave pass, 2048-edge tiles): 83 MB of DRAM traffic (the 62 MB '
                 'of stored edge lists and the candidates\' records); long-scoreboard stalls dominate'},
 }
@@ -357,7 +358,7 @@ def gpu_arm(args, world, rank):
     totals = {k: float(np.sum(v)) for k, v in kt.items()}
     dom = max(totals, key=totals.get)
     roofline = roofline_block(dom, totals, kt, sim, n, st, res)
-    launches_per_step = 1 + 4 * npts + 1  # seed infect, per day agent/stored/dynamic/infect, closing pass
+    launches_per_step = 2 + 4 * npts + 1  # rewind copies, seed infect, per day agent/stored/dynamic/infect, closing pass
 
     # end to end through the public API, from pinned host memory
     e2e = None

@@ -1151,14 +1151,14 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_edge_pass_res(covgpu_state s
 // sources, not the layer's edges: a quiet day costs a read of the source bitmap.
 constexpr int DYN_WARPS = 8;  // warps per thread block
 // Warps per agent block of the per-source passes (split: each warp takes 8 / split
-// of the agent block's eight source-bitmap words): one from SPLIT_TARGET agent
-// blocks up, else doubled until that many warps. A warp's set-up is a chain of
-// about six dependent loads, so more warps only pay where the chip would idle: the
-// 1M-agent run took 15.9 ms with one, 16.5 with two, 17.7 with four and 20.0 with
-// eight; 300,000 agents 7.0 ms with two (7.2 with one), 7.3 with four, 7.6 with
-// eight; 100,000 agents the same (8.1 ms) with four and eight.
+// of the agent block's eight source-bitmap words): doubled until there are
+// SPLIT_TARGET warps, about ten an SM. A warp's set-up is a chain of about six
+// dependent loads, so more warps only pay where the chip would idle (ms a 100-day run
+// with one / two / four / eight: 20,000 agents 3.19, 3.00, 2.86, 2.79; 100,000 3.30,
+// 3.11, 3.09, 3.25; 200,000 4.15, 3.99, 3.99, -; 300,000 with testing, 120 days, 6.82,
+// 6.56, -, -; 1M, 180 days, 14.9, 15.5, 17.7, 20.0).
 constexpr int AB_WORDS = AGENT_THREADS / 32;  // source-bitmap words of an agent block
-constexpr int64_t SPLIT_TARGET = 2048;
+constexpr int64_t SPLIT_TARGET = 1520;
 inline int source_split(const covgpu_state* st) {
   int split = 1;
   while (split < AB_WORDS && st->n_agent_blocks * split < SPLIT_TARGET) split *= 2;
