@@ -244,7 +244,7 @@ def kernel_profile(sim, npts, head_start_cycles=2_000_000):
     return {k: [a.elapsed_time(b) for a, b in v] for k, v in times.items()}
 
 
-KERNEL_NAMES = {'agent_step': 'k_agent_step', 'edge_stored': 'k_edge_pass', 'edge_dynamic': 'k_dyn_pass',
+KERNEL_NAMES = {'agent_step': 'k_agent_step', 'edge_stored': 'k_edge_pass', 'edge_dynamic': 'k_source_pass',
                 'infect_claims': 'k_infect_claims'}
 
 

@@ -975,7 +975,7 @@ __device__ __forceinline__ void lik_flush_warp(const covgpu_state& st, int t, in
 
 // Stored layers on quiet days. A stored layer segment with an agent index (rp1,
 // rp2, perm2: each agent's edges as p1 and as p2) is walked from the day's
-// sources (k_src_pass) instead of streamed edge by edge (the tile passes) while
+// sources (walk_body) instead of streamed edge by edge (the tile passes) while
 // its sim's infectious agents times st.src_walk are fewer than its agents (0:
 // never, -1: always): the number infectious at the end of day t-1 plus day t's
 // new infectious, less its recoveries and deaths, from the results the agent
