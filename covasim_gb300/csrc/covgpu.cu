@@ -915,23 +915,22 @@ __device__ __forceinline__ void edge_tile(const covgpu_state& st, int t, int seg
   }
 }
 
-// Tiles [k_lo, k_hi) of one stored segment (L, its sim's constants sp) as one
-// stream of rounds: each round's edge lists are loaded one round ahead, across
-// the tiles' boundaries, and the warp's queue entries count edges from a base
+// Units [k_lo, k_hi) of UNIT edges of one stored segment (L, its sim's constants sp) as
+// one stream: each round's edge lists are loaded one round ahead, and the warp's queue entries count edges from a base
 // that moves on (the queue drained first) when a round would reach past the
 // 2^15 edges their offsets hold.
-template <bool LIK, int64_t TILE>
+template <bool LIK, int64_t UNIT>
 __device__ __forceinline__ void edge_span(const covgpu_state& st, int t, int seg, int64_t k_lo, int64_t k_hi,
                                           const covgpu_layer* L, const SimLite* sp, EdgeQueue& q, LikAcc& acc) {
   constexpr int64_t ROUND = (int64_t)EDGE_THREADS * EDGE_VEC;
   constexpr int64_t SPAN = 32768;
-  static_assert(TILE % ROUND == 0 && SPAN % ROUND == 0, "whole rounds");
+  static_assert(UNIT % ROUND == 0 && SPAN % ROUND == 0, "whole rounds");
   SegCtx c;
   seg_ctx(st, t, seg, L, sp, c);
   const int32_t* p1 = L->p1;
   const int32_t* p2 = L->p2;
-  const int64_t e_lo = k_lo * TILE;
-  const int64_t e_hi = min(k_hi * TILE, c.n_edges);
+  const int64_t e_lo = k_lo * UNIT;
+  const int64_t e_hi = min(k_hi * UNIT, c.n_edges);
   const int32_t off = (int32_t)sp->agent_off;
   auto fetch = [&](int64_t rb, int4& xa, int4& xb) {
     const int64_t eb = rb + (int64_t)threadIdx.x * EDGE_VEC;
@@ -1034,25 +1033,30 @@ __global__ void __launch_bounds__(EDGE_THREADS) k_edge_pass(covgpu_state st, int
 }
 
 // The stored layers as one wave of resident blocks (covgpu_state.edge_wave): of the
-// T tiles, block b walks [b T / G, (b + 1) T / G), a contiguous share that differs
-// from the others' by at most one tile, segment by segment, its edge lists loaded a
-// round ahead across the tiles' boundaries. Against one block per tile it leaves
-// no partial last wave and no per-tile start (segment lookup, first round's
-// latency); the tile size only sets how finely the shares are balanced.
-template <bool LIK, int ROUNDS>
+// U units of all tiles, block b streams [b U / G, (b + 1) U / G), a contiguous share
+// that differs from the others' by at most one unit, segment by segment, its edge
+// lists loaded a round ahead across the tiles' boundaries. Against one block per tile
+// it leaves no partial last wave and no per-tile start (segment lookup, first round's
+// latency). FINE: a unit is a round instead of a tile, which gives small states more
+// blocks (60,000 agents 1.55 -> 1.44 ms a 60-day run); not beside a redrawn layer's pass
+// on the side stream, whose blocks need the SMs' room too (100,000 agents with the
+// likelihood 7.9 -> 8.4 ms).
+template <bool LIK, int ROUNDS, bool FINE>
 __global__ void __launch_bounds__(EDGE_THREADS) k_edge_wave(covgpu_state st, int t) {
-  constexpr int64_t TILE = (int64_t)ROUNDS * EDGE_ROUND;
-  const int64_t lo = st.n_tiles * (int64_t)blockIdx.x / gridDim.x;
-  const int64_t hi = st.n_tiles * ((int64_t)blockIdx.x + 1) / gridDim.x;
+  constexpr int PER = FINE ? ROUNDS : 1;  // units per tile
+  constexpr int64_t UNIT = (int64_t)ROUNDS * EDGE_ROUND / PER;
+  const int64_t units = st.n_tiles * PER;
+  const int64_t lo = units * (int64_t)blockIdx.x / gridDim.x;
+  const int64_t hi = units * ((int64_t)blockIdx.x + 1) / gridDim.x;
   if (lo >= hi) return;  // block-uniform
   __shared__ covgpu_layer s_L;
   __shared__ SimLite s_sp;
   __shared__ EdgeQueue s_q[EDGE_THREADS / 32];
   __shared__ double s_acc[EDGE_THREADS / 32][2];
-  int seg = segment_of_tile(st.segments, st.n_segments, lo);  // the segment table is read-only
+  int seg = segment_of_tile(st.segments, st.n_segments, lo / PER);  // the segment table is read-only
   pdl_wait();
   if (held(st, t)) return;
-  int64_t tile = lo;
+  int64_t unit = lo;
   for (;;) {
     if (threadIdx.x == 0) {
       s_L = st.segments[seg];
@@ -1060,11 +1064,11 @@ __global__ void __launch_bounds__(EDGE_THREADS) k_edge_wave(covgpu_state st, int
     }
     __syncthreads();
     const int64_t seg_end = seg + 1 < st.n_segments ? st.segments[seg + 1].tile_begin : st.n_tiles;
-    const int64_t stop = min(hi, seg_end);  // >= tile: seg is the last segment starting at or before tile
-    if (tile < stop && !seg_walked(st, s_L, t)) {  // block-uniform
+    const int64_t stop = min(hi, seg_end * PER);  // >= unit: seg is the last segment starting at or before it
+    if (unit < stop && !seg_walked(st, s_L, t)) {  // block-uniform
       LikAcc acc;
-      edge_span<LIK, TILE>(st, t, seg, tile - s_L.tile_begin, stop - s_L.tile_begin, &s_L, &s_sp,
-                           s_q[threadIdx.x >> 5], acc);
+      const int64_t begin = s_L.tile_begin * PER;
+      edge_span<LIK, UNIT>(st, t, seg, unit - begin, stop - begin, &s_L, &s_sp, s_q[threadIdx.x >> 5], acc);
       if (LIK) {  // this segment's sums: one sim, one layer
         const double a = warp_sum_d(ff_to_d(acc.ll)), b = warp_sum_d(ff_to_d(acc.g));
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1080,8 +1084,8 @@ __global__ void __launch_bounds__(EDGE_THREADS) k_edge_wave(covgpu_state st, int
         }
       }
     }
-    if (stop > tile) tile = stop;
-    if (tile >= hi || seg + 1 >= st.n_segments) break;
+    if (stop > unit) unit = stop;
+    if (unit >= hi || seg + 1 >= st.n_segments) break;
     ++seg;
     __syncthreads();  // every thread has read s_L (and s_acc) before they are replaced
   }
@@ -1697,24 +1701,28 @@ int configure_edge_pass(const covgpu_state* st) {
   return rc ? rc : configure_res<true>(smem);
 }
 
-// one wave of k_edge_wave<LIK, R>: at most st->edge_wave blocks per SM
-template <bool LIK, int R>
+// one wave of k_edge_wave<LIK, R, FINE>: at most st->edge_wave blocks per SM
+template <bool LIK, int R, bool FINE>
 void launch_edge_wave_r(const covgpu_state* st, int t, cudaStream_t s) {
-  static int64_t per_sm = -1;
-  if (per_sm < 0) per_sm = wave_blocks(k_edge_wave<LIK, R>, EDGE_THREADS) / n_sms();
+  static const int64_t per_sm = wave_blocks(k_edge_wave<LIK, R, FINE>, EDGE_THREADS) / n_sms();
   const int64_t wave = (int64_t)n_sms() * (st->edge_wave < per_sm ? st->edge_wave : per_sm);
-  const unsigned grid = (unsigned)(st->n_tiles < wave ? st->n_tiles : wave);
-  launch_pdl(k_edge_wave<LIK, R>, grid, EDGE_THREADS, 0, s, *st, t);
+  const int64_t units = st->n_tiles * (FINE ? R : 1);
+  launch_pdl(k_edge_wave<LIK, R, FINE>, (unsigned)(units < wave ? units : wave), EDGE_THREADS, 0, s, *st, t);
+}
+template <bool LIK, int R>
+void launch_edge_wave(const covgpu_state* st, int t, cudaStream_t s) {
+  if (st->n_dynamic == 0) launch_edge_wave_r<LIK, R, true>(st, t, s);
+  else launch_edge_wave_r<LIK, R, false>(st, t, s);
 }
 
 template <bool LIK>
 void launch_edge_tiles(const covgpu_state* st, int t, cudaStream_t s) {
   if (st->edge_wave > 0) {
     switch (st->edge_tile) {
-      case 1024: launch_edge_wave_r<LIK, 1>(st, t, s); break;
-      case 2048: launch_edge_wave_r<LIK, 2>(st, t, s); break;
-      case 8192: launch_edge_wave_r<LIK, 8>(st, t, s); break;
-      default: launch_edge_wave_r<LIK, 4>(st, t, s); break;
+      case 1024: launch_edge_wave<LIK, 1>(st, t, s); break;
+      case 2048: launch_edge_wave<LIK, 2>(st, t, s); break;
+      case 8192: launch_edge_wave<LIK, 8>(st, t, s); break;
+      default: launch_edge_wave<LIK, 4>(st, t, s); break;
     }
     return;
   }
