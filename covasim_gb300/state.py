@@ -277,11 +277,13 @@ def ili_agents(seed, t, n, n_ili):
 #   4.19; 300,000 5.23, 5.06, 5.46; 1M 10.97, 9.24, 9.69; 4M 18.0, 10.2, 10.3);
 # * several: every day (24 to 96 random sims, streamed / every day / 1/64: 17M edges
 #   16.0, 18.1, 16.9; 30M 24.6, 24.6, 24.6; 43M 33.1, 29.2, 31.7; 115M -, 83.5, 106);
-# * a redrawn layer and testing, below SRC_WALK_ALL_AGENTS agents: walked every day,
-#   one launch with the redrawn layer's pass instead of a fork and join of two (ms a
-#   120-day run, every day / below 1/16 / below 1/128: 200,000 agents 6.40, 6.76, 6.57;
-#   300,000 6.85, 7.25, 7.15; 600,000 9.32, 9.74, 9.39); above, below 1/16 (10M with
-#   three variants 105.2, 105.4, 111.3);
+# * a redrawn layer and testing: one sim walks every day, one launch with the redrawn
+#   layer's pass instead of a fork and join of two (100-120 days, every day / 1/16 /
+#   1/128: 200,000 agents 6.40, 6.76, 6.57; 300,000 6.85, 7.25, 7.15; 800,000 8.83, 9.10,
+#   8.79; 1.5M 12.97, 13.30, 13.72; 6M, 60 days, 15.8, 15.9, 16.5; 10M, three variants,
+#   105.2, 105.4, 111.3); several do below SRC_WALK_ALL_AGENTS agents, else SRC_WALK
+#   (16 of 20,000 7.12, 7.45, 7.30; 8 of 60,000 7.91, 8.25, 7.87; 48 of 20,000 12.9,
+#   13.3, 12.6);
 # * a redrawn layer without testing: below 1/32, the stream beside the redrawn layer's
 #   pass being faster on the busy days (every day / 1/16 / 1/32 / 1/128: 30,000 agents
 #   3.51, 3.43, 3.41, 3.38; 300,000 5.75, 5.59, 5.55, 5.55; 1M, 150 days, 14.75, 13.25,
@@ -289,9 +291,8 @@ def ili_agents(seed, t, n, n_ili):
 # * with the likelihood, whose walk takes the layers one after another, SRC_WALK
 #   (100,000 agents: 7.96 ms, 8.44 every day).
 SRC_WALK = 128
-SRC_WALK_TESTING = 16
 SRC_WALK_REDRAWN = 32
-SRC_WALK_ALL_AGENTS = 600_000
+SRC_WALK_ALL_AGENTS = 400_000
 SRC_WALK_BIG = 64
 SRC_WALK_MIN_EDGES = 10_000_000
 SRC_WALK_MIN_EDGES_BATCH = 30_000_000
@@ -787,7 +788,7 @@ class BatchState:
         if self._walk_default and indexed and not self.lik_active:
             dynamic = any(rec.dynamic for rec in self.segments)
             if dynamic and self.has_testing:
-                k = -1 if self.n < SRC_WALK_ALL_AGENTS else SRC_WALK_TESTING
+                k = -1 if len(self.specs) == 1 or self.n < SRC_WALK_ALL_AGENTS else SRC_WALK
             elif dynamic:
                 k = SRC_WALK_REDRAWN
             elif len(self.specs) > 1:
