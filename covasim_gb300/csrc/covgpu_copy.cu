@@ -54,7 +54,9 @@ __global__ void __launch_bounds__(COPY_THREADS) k_copy_spans(const __grid_consta
 
 // sim.py:920-932: per block, the number of outcomes (recoveries and deaths), the sum
 // of their dates and the sum of those agents' infectious dates (float64, each thread
-// over its agents in order, then a tree: the same for every run)
+// over its agents in order, then a tree: the same for every run). A barrier after each
+// step of the tree, the last one included: its sums are stored by other threads of the
+// warp than the one that formed them.
 constexpr int SUM_THREADS = 256;
 __global__ void __launch_bounds__(SUM_THREADS) k_outcome_sums(const float* __restrict__ rec,
                                                               const float* __restrict__ dead,
@@ -70,10 +72,11 @@ __global__ void __launch_bounds__(SUM_THREADS) k_outcome_sums(const float* __res
   s[0][threadIdx.x] = cnt;
   s[1][threadIdx.x] = s_out;
   s[2][threadIdx.x] = s_inf;
+  __syncthreads();
   for (int o = SUM_THREADS / 2; o > 0; o >>= 1) {
-    __syncthreads();
     if (threadIdx.x < o)
       for (int k = 0; k < 3; ++k) s[k][threadIdx.x] += s[k][threadIdx.x + o];
+    __syncthreads();
   }
   if (threadIdx.x < 3) out[3 * (int64_t)blockIdx.x + threadIdx.x] = s[threadIdx.x][0];
 }
