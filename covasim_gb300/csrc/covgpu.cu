@@ -563,11 +563,11 @@ __global__ void __launch_bounds__(AGENT_THREADS, QUEUE ? AGENT_QUEUE_BLOCKS : AG
 // source bit (infectious with a variant and rel_trans != 0) and target bit
 // (susceptible with rel_sus != 0) of agent a: two separate bitmaps, so that the
 // source bitmap (n/8 bytes), tested for both endpoints of every edge, stays in L1
-__device__ __forceinline__ uint32_t src_bit(const uint32_t* __restrict__ roles, int32_t a) {
+__device__ __forceinline__ uint32_t src_bit(const uint32_t* roles, int32_t a) {
   return (ld_keep_u32(roles + (a >> 5)) >> (a & 31)) & 1u;
 }
 __device__ __forceinline__ uint32_t tgt_bit(const covgpu_state& st, int32_t a) {
-  return (__ldg(st.roles + roles_words(st) + (a >> 5)) >> (a & 31)) & 1u;
+  return (st.roles[roles_words(st) + (a >> 5)] >> (a & 31)) & 1u;
 }
 
 // per-tile constants, hoisted out of the segment and sim records
@@ -652,7 +652,7 @@ __device__ __forceinline__ void lik_terms(const covgpu_state& st, const SegCtx& 
 template <bool LIK, bool INJ = true, bool THIN = false>
 __device__ __forceinline__ bool edge_try(const covgpu_state& st, const SegCtx& c, int t, int64_t e, int dir,
                                          int32_t s, int32_t g, uint32_t& v_out, LikAcc& acc, bool ph = true) {
-  const float4 sr = __ldg(reinterpret_cast<const float4*>(st.src_rec) + s);
+  const float4 sr = reinterpret_cast<const float4*>(st.src_rec)[s];
   const uint32_t fs = __float_as_uint(sr.w);
   const float lb = c.edge_beta ? __ldg(c.edge_beta + e) : c.beta_const;
   const float rt = sr.x, vl = sr.y;
@@ -662,14 +662,14 @@ __device__ __forceinline__ bool edge_try(const covgpu_state& st, const SegCtx& c
   const float beta = __ldg(c.beta_t + vc);
   // the target: its record (rel_sus * (1 - sus_imm), sign bit = quarantined); the
   // quarantined, and the likelihood's terms, take the fields themselves
-  const uint32_t tr = __float_as_uint(__ldg(st.tgt_rec + gv));
+  const uint32_t tr = __float_as_uint(st.tgt_rec[gv]);
   const bool tquar = tr >> 31;
   uint32_t fg = tquar ? B_QUAR : 0u;
   float rs = 0.0f, si = 0.0f;
   if (LIK || tquar) {
-    fg = __ldg(st.flags + g);
-    rs = __ldg(st.rel_sus + g);
-    si = __ldg(st.sus_imm + gv);
+    fg = st.flags[g];
+    rs = st.rel_sus[g];
+    si = st.sus_imm[gv];
   }
   if (v >= (uint32_t)c.nv) return false;
   float rte = rt;
@@ -993,9 +993,12 @@ __device__ __forceinline__ bool seg_walked(const covgpu_state& st, const covgpu_
   return inf * (int64_t)st.src_walk < sp.n_agents;
 }
 
-// One block per tile (none for a segment walked from its sources today).
+// One block per tile (none for a segment walked from its sources today). The bound
+// here and at k_edge_wave keeps the registers (48, with the likelihood 62) and so the
+// resident blocks an SM: with the lookups as plain loads the compiler would take 64
+// and 54, one block fewer.
 template <bool LIK, int ROUNDS>
-__global__ void __launch_bounds__(EDGE_THREADS) k_edge_pass(covgpu_state st, int t) {
+__global__ void __launch_bounds__(EDGE_THREADS, LIK && ROUNDS >= 4 ? 5 : 0) k_edge_pass(covgpu_state st, int t) {
   pdl_wait();
   if (held(st, t)) return;
   constexpr int64_t TILE = (int64_t)ROUNDS * EDGE_ROUND;
@@ -1042,7 +1045,7 @@ __global__ void __launch_bounds__(EDGE_THREADS) k_edge_pass(covgpu_state st, int
 // on the side stream, whose blocks need the SMs' room too (100,000 agents with the
 // likelihood 7.9 -> 8.4 ms).
 template <bool LIK, int ROUNDS, bool FINE>
-__global__ void __launch_bounds__(EDGE_THREADS) k_edge_wave(covgpu_state st, int t) {
+__global__ void __launch_bounds__(EDGE_THREADS, LIK ? 4 : 5) k_edge_wave(covgpu_state st, int t) {
   constexpr int PER = FINE ? ROUNDS : 1;  // units per tile
   constexpr int64_t UNIT = (int64_t)ROUNDS * EDGE_ROUND / PER;
   const int64_t units = st.n_tiles * PER;
@@ -1120,8 +1123,8 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_edge_pass_res(covgpu_state s
   if (!streamed) return;  // block-uniform
   // bitmap words four at a time (the bitmap has room for whole uint4s)
   const uint4* g4 = reinterpret_cast<const uint4*>(st.roles);
-  for (int64_t k = threadIdx.x; k < (words >> 2); k += RES_THREADS) s_dyn[k] = __ldg(g4 + k);
-  for (int64_t k = (words & ~3ll) + threadIdx.x; k < words; k += RES_THREADS) s_src[k] = __ldg(st.roles + k);
+  for (int64_t k = threadIdx.x; k < (words >> 2); k += RES_THREADS) s_dyn[k] = g4[k];
+  for (int64_t k = (words & ~3ll) + threadIdx.x; k < words; k += RES_THREADS) s_src[k] = st.roles[k];
   if (threadIdx.x == 0) load_sim_lite(s_sp, st.sims[0]);
   EdgeQueue* s_q = reinterpret_cast<EdgeQueue*>(s_dyn + ((words + 3) >> 2));
   EdgeQueue& q = s_q[threadIdx.x >> 5];
@@ -1194,7 +1197,7 @@ __device__ __forceinline__ void dyn_ctx(const covgpu_state& st, const covgpu_sim
 // lb * rel_trans'(s) * rse_max, formed as edge_try forms p; -1 when the source
 // cannot transmit in this layer
 __device__ __forceinline__ int dyn_shift(const covgpu_state& st, const SegCtx& c, int32_t s) {
-  const float4 sr = __ldg(reinterpret_cast<const float4*>(st.src_rec) + s);
+  const float4 sr = reinterpret_cast<const float4*>(st.src_rec)[s];
   const uint32_t fs = __float_as_uint(sr.w);
   const uint32_t v = (__float_as_uint(sr.z) >> 8) & 0xFFu;
   if (v >= (uint32_t)c.nv) return -1;
@@ -1270,7 +1273,7 @@ __device__ __forceinline__ void dyn_body(const covgpu_state& st, int t, int64_t 
   const int64_t w0 = (blk.begin >> 5) + w_lo;  // sims start at multiples of 32
   pdl_wait();
   if (held(st, t)) return;
-  const WarpBits wb = warp_bits_scan(lane < nw ? __ldg(st.roles + w0 + lane) : 0u);
+  const WarpBits wb = warp_bits_scan(lane < nw ? st.roles[w0 + lane] : 0u);
   if (wb.total == 0) return;
   const covgpu_sim_params& sp = st.sims[blk.sim];
   const uint32_t n_local = (uint32_t)sp.n_agents, thr = bounded_thr(n_local);
@@ -1479,7 +1482,7 @@ __device__ __forceinline__ void walk_body(const covgpu_state& st, int t, int64_t
   }
   pdl_wait();
   if (held(st, t)) return;
-  const WarpBits wb = warp_bits_scan(lane < nw ? __ldg(st.roles + w0 + lane) : 0u);
+  const WarpBits wb = warp_bits_scan(lane < nw ? st.roles[w0 + lane] : 0u);
   if (wb.total == 0) return;
   walked = walked && seg_walked(st, st.segments[seg], t);
   const unsigned mask = __ballot_sync(0xffffffffu, walked);  // the walked layers

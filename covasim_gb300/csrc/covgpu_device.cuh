@@ -227,9 +227,12 @@ __device__ __forceinline__ int64_t uniform_index(uint32_t a, uint32_t b, uint64_
   return (int64_t)__umul64hi(x, n);
 }
 // ---------------------------------------------------------------- small helpers
-// Read-only global loads with an L1 policy (the data is not written while the
-// kernel runs). COVGPU_L1_HINTS selects them: bit 0 keeps the source bitmap in
-// L1 (evict_last), bit 1 streams the edge lists past L1 (no_allocate). L2
+// Global loads with an L1 policy. COVGPU_L1_HINTS selects them: bit 0 keeps the
+// source bitmap in L1 (evict_last), bit 1 streams the edge lists, which no kernel
+// writes, past L1 (no_allocate, read-only). Arrays that a day's kernels write (the
+// role bitmaps, the records, the agents' fields) are read with plain loads: a kernel
+// launched as a dependent can be resident while its predecessor still writes them,
+// and the read-only path is only for data constant over the kernel's life. L2
 // policy is the default: the edge lists stay L2-resident from day to day.
 // Streaming the edge lists past L1 shortened a 1M-agent, 180-day run by 7%
 // (the agent and infect passes gained most); sending the candidates' agent
@@ -250,10 +253,10 @@ __device__ __forceinline__ int4 ld_stream_v4(const int32_t* p) {
 __device__ __forceinline__ uint32_t ld_keep_u32(const uint32_t* p) {
 #if COVGPU_L1_HINTS & 1
   uint32_t v;
-  asm("ld.global.nc.L1::evict_last.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  asm volatile("ld.global.L1::evict_last.u32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
 #else
-  return __ldg(p);
+  return *p;
 #endif
 }
 

@@ -47,10 +47,11 @@ inline unsigned wave_grid(const covgpu_state* st, int64_t wave) {
 
 // Programmatic dependent launch: a kernel launched with
 // launch_pdl may be scheduled while its stream predecessor's last blocks finish
-// (inside a captured graph the edge becomes a programmatic one); pdl_wait, the
-// first statement of each such kernel, holds it until the predecessor has
-// completed and its writes are visible. Launched the ordinary way, pdl_wait
-// returns at once.
+// (inside a captured graph the edge becomes a programmatic one); pdl_wait
+// holds it until the predecessor has completed and its writes are visible.
+// Before it a kernel reads only what no kernel writes: the sim, segment and
+// agent-block tables, the layers' records, constant tables. Launched the
+// ordinary way, pdl_wait returns at once.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // A block's signal that the next kernel's blocks may be scheduled once every block
 // of this grid has given it or exited: their set-up before pdl_wait (tables,

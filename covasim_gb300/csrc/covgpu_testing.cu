@@ -415,8 +415,8 @@ __global__ void __launch_bounds__(AGENT_THREADS) k_trace_marks(covgpu_state st, 
   mark_block(st, t, s_list);
 }
 
-__device__ __forceinline__ uint32_t bit_of(const uint32_t* __restrict__ bits, int32_t a) {
-  return (__ldg(bits + (a >> 5)) >> (a & 31)) & 1u;
+__device__ __forceinline__ uint32_t bit_of(const uint32_t* bits, int32_t a) {
+  return (bits[a >> 5] >> (a & 31)) & 1u;
 }
 
 // contact_tracing.identify_contacts, the find_contacts half (utils.py:131-147):
