@@ -244,8 +244,9 @@ __device__ __forceinline__ void test_flush(const covgpu_state& st, int t, int si
   tested_acc = 0;
 }
 
-// The per-sim preparation of day t's test pass, one block per sim:
-// test_prob's swab-delay histogram is cleared (k_swab_hist fills it), and the
+// The per-sim preparation of day t's test pass, one block per sim: the count of the
+// day's traced cases is cleared (on every day: cases with a delayed diagnosis are traced
+// after test_prob's last day), test_prob's swab-delay histogram is cleared (k_swab_hist fills it), and the
 // day's influenza-like illnesses (interventions.py:941-947), drawn on the host
 // (they do not depend on the state), are marked with t.
 __global__ void k_test_prep(covgpu_state st, int t) {
@@ -253,10 +254,10 @@ __global__ void k_test_prep(covgpu_state st, int t) {
   const int s = blockIdx.x;
   if (s >= st.n_sims) return;
   const covgpu_testing& T = st.sims[s].testing;
+  if (T.cap_list && threadIdx.x == 0) *T.cap_count = 0u;
   if (!day_active(t, T.test_start, T.test_end)) return;
   if (T.swab_pdf)
     for (int k = threadIdx.x; k <= T.swab_len; k += blockDim.x) T.swab_bins[k] = 0;
-  if (T.cap_list && threadIdx.x == 0) *T.cap_count = 0u;
   if (!T.ili_mark) return;
   const int d = t - T.test_start;
   if (d < 0 || d >= T.ili_days) return;
