@@ -55,11 +55,11 @@ constexpr int IMPORT_BLOCKS = 4;       // k_import_day grid (a day imports a han
 
 
 // Fixed-point terms of the levels' sums, by 32-bit conversions (64-bit ones run at
-// the float64 rate, 16 cycles a warp): x * 2^24 of a NAb level (at least 128: the
-// 64-bit conversion), and x * 2^32 of an efficacy in [0, 1] (1 saturates).
+// the float64 rate, 16 cycles a warp): x * 2^24 of a NAb level (128 or more of either
+// sign, or NaN: the 64-bit conversion), and x * 2^32 of an efficacy in [0, 1] (1 saturates).
 __device__ __forceinline__ long long nab_fixed(float x) {
   const float y = __fmul_rn(x, 16777216.0f);
-  return y < 2147483648.0f ? (long long)__float2int_rn(y) : __float2ll_rn(y);
+  return fabsf(y) < 2147483648.0f ? (long long)__float2int_rn(y) : __float2ll_rn(y);
 }
 __device__ __forceinline__ long long efficacy_fixed(float x) {
   return (long long)__float2uint_rn(__fmul_rn(x, 4294967296.0f)) + (x >= 1.0f ? 1 : 0);
