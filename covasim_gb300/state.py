@@ -1248,16 +1248,22 @@ class BatchState:
 
     def _spans(self, copies, zeros=(), ones=()):
         """Copy each (dst, src) pair, zero each of ``zeros`` and set every bit of each
-        of ``ones`` in one launch (covgpu_copy_spans); pairs that are not plain
-        copies (another type, size, layout or device) go through ``copy_``."""
-        todo, dev = [], self.res_all.device
+        of ``ones`` in one launch (covgpu_copy_spans). Pairs that are not plain copies
+        on the state's device (another type, size, layout or device on either side) go
+        through ``copy_`` before it, and so do those whose destination is then cleared
+        and, all of them, copies among the destinations: the launch writes every array
+        once, in no order."""
+        dev = self.res_all.device
+        todo = [(x, None, 0) for x in zeros] + [(x, None, 0xFF) for x in ones]
+        cleared, written = {x.data_ptr() for x, _, _ in todo}, {dst.data_ptr() for dst, _ in copies}
+        ordered = any(src.data_ptr() in written for _, src in copies)
         for dst, src in copies:
-            if (type(src) is torch.Tensor and src.dtype == dst.dtype and src.shape == dst.shape and
-                    src.device == dev and dst.is_contiguous() and src.is_contiguous()):
+            if (not ordered and type(src) is torch.Tensor and type(dst) is torch.Tensor and src.dtype == dst.dtype and
+                    src.shape == dst.shape and src.device == dev and dst.device == dev and dst.is_contiguous() and
+                    src.is_contiguous() and not src.is_neg() and not dst.is_neg() and dst.data_ptr() not in cleared):
                 todo.append((dst, src.data_ptr(), 0))
             else:
                 dst.copy_(src)
-        todo += [(x, None, 0) for x in zeros] + [(x, None, 0xFF) for x in ones]
         spans = (L.Span * len(todo))(*((x.data_ptr(), src, x.numel() * x.element_size(), fill, 0)
                                        for x, src, fill in todo))
         L.call('covgpu_copy_spans', spans, len(todo), _stream())
