@@ -68,8 +68,12 @@ def mean_infectious_duration(d_rec, d_dead, d_inf):
     """sim.py:920-932: mean of the outcome dates minus mean of the infectious dates,
     over the agents with a recovery date then those with a death date (numpy
     arrays or device tensors; sums in float64)."""
-    if torch.is_tensor(d_rec) and not all(x.is_cuda and x.dtype == torch.float32 for x in (d_rec, d_dead, d_inf)):
-        d_rec, d_dead, d_inf = (x.cpu().numpy() for x in (d_rec, d_dead, d_inf))
+    if torch.is_tensor(d_rec):
+        if not d_rec.shape == d_dead.shape == d_inf.shape:  # the kernel reads all three to the first one's length
+            raise IndexError('mean_infectious_duration: the dates are of different lengths')
+        d_rec, d_dead, d_inf = (x.resolve_neg() for x in (d_rec, d_dead, d_inf))
+        if not all(x.is_cuda and x.dtype == torch.float32 and x.device == d_rec.device for x in (d_rec, d_dead, d_inf)):
+            d_rec, d_dead, d_inf = (x.cpu().numpy() for x in (d_rec, d_dead, d_inf))
     if torch.is_tensor(d_rec):  # per-block sums on the device, one read-back
         d_rec, d_dead, d_inf = (x.contiguous() for x in (d_rec, d_dead, d_inf))
         if not d_rec.numel():
