@@ -25,6 +25,7 @@ N_RES_F = 3
 FX_NAB_BITS = 24
 FX_IMM_BITS = 32
 NO_VARIANT = 0xFF
+ABI_VERSION = 2  # COVGPU_VERSION
 WALK_ALL = -(1 << 31)  # covgpu_state.src_walk: every stored layer walked every day (COVGPU_WALK_ALL)
 NOALLOC_MAX_EDGES = 1 << 24   # covgpu_infections_noalloc limit (COVGPU_NOALLOC_MAX_EDGES)
 NO_SUBTARGET = 0xFFFFFFFFFFFFFFFF  # covgpu_testing.sub_thr: no subtarget (COVGPU_NO_SUBTARGET)

@@ -2549,7 +2549,7 @@ int check_state(const covgpu_state* st) {
 
 extern "C" {
 
-int covgpu_version(void) { return 1; }
+int covgpu_version(void) { return COVGPU_VERSION; }
 
 int covgpu_abi_layout(int64_t* out, int32_t n) {
   const int64_t v[] = {(int64_t)sizeof(covgpu_sim_params), (int64_t)sizeof(covgpu_layer),

@@ -716,7 +716,10 @@ int covgpu_update_peak_nab(const covgpu_state* st, int32_t t, int32_t sim, const
                            const int8_t* symp_class, covgpu_dur_par nab_init, float nab_boost, double norm_factor,
                            int32_t call_tag, void* stream);
 
-/* Library/ABI version. */
+/* Library/ABI version: COVGPU_VERSION of the header the library was built with. A
+ * caller whose header has another one lays the structures out differently. 2:
+ * covgpu_layer has rev1, covgpu_sim_params dur_ff and dur_int. */
+#define COVGPU_VERSION 2
 int covgpu_version(void);
 
 /* ABI layout check (no device work): writes up to n values: sizeof of
