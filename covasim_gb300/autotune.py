@@ -28,11 +28,13 @@ _CACHE = {}
 
 
 def workload_signature(state):
-    """Edge counts per (stored, dynamic) layer kind, agents, sims, and the device."""
+    """Edge counts per (stored, dynamic) layer kind, agents, sims, the device, and what
+    decides on which days the stored layers' pass runs and beside what."""
     stored = sum(int(r.n_edges) for r in state.segments if not r.dynamic)
     dynamic = sum(int(r.n_edges) for r in state.segments if r.dynamic)
     name = torch.cuda.get_device_name(state.device)
-    return f'{name}|n={state.n}|sims={len(state.specs)}|stored={stored}|dynamic={dynamic}'
+    return (f'{name}|n={state.n}|sims={len(state.specs)}|stored={stored}|dynamic={dynamic}'
+            f'|walk={state.cstate.src_walk}|testing={int(state.has_testing)}|lik={int(state.lik_active)}')
 
 
 def _one_run(state, snap, t1):
@@ -57,7 +59,10 @@ def tune_edge_tile(state, days=None, candidates=L.EDGE_TILES, reps=2, cache_file
     shared memory, timed over ``reps`` whole runs of ``days`` days (default: all).
     Leaves the state rewound with the best variant set. Returns (best label,
     {label: ms per run}); a label is the tile size, suffixed 'w' for the one-wave
-    pass and 'r' for the resident variant."""
+    pass and 'r' for the resident variant. A state that never launches the pass
+    (src_walk COVGPU_WALK_ALL) keeps its choice, untimed: (its label, {})."""
+    if state.cstate.src_walk == L.WALK_ALL:
+        return str(state.edge_tile_label), {}
     key = workload_signature(state) + f'|days={days}'
     if cache_file and os.path.exists(cache_file) and key not in _CACHE:
         with open(cache_file) as f:
