@@ -26,7 +26,10 @@ def _ptr(t):
 
 
 def _raw_stream(x):
-    return torch._C._cuda_getCurrentRawStream(x.get_device())
+    try:
+        return torch._C._cuda_getCurrentRawStream(x.get_device())
+    except AttributeError:  # a private name: the public way takes a microsecond more
+        return torch.cuda.current_stream(x.device).cuda_stream
 
 
 def _direct(xs, dtypes, *ints):
@@ -36,16 +39,22 @@ def _direct(xs, dtypes, *ints):
     compilation, profiling, gradients) and every argument is a plain contiguous
     tensor of the current device in one of its dtypes (and the integers fit the
     operators' int64). The operators' Python machinery takes about 30 us a call:
-    the viral load of 20,000 agents took 45.7 us through them and takes 14.2 us."""
-    if (torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack() or
-            torch._C._get_tracing_state() is not None or torch.compiler.is_compiling() or
-            torch._C._functorch.peek_interpreter_stack() is not None or
-            torch.autograd.forward_ad._current_level >= 0 or torch._C._autograd._profiler_enabled()):
+    the viral load of 20,000 agents took 45.7 us through them and takes 14.2 us.
+    torch's own (private) names are asked; without one of them the answer is no."""
+    if torch.compiler.is_compiling():  # first: constant under compilation, which knows none of the names below
+        return False
+    try:
+        if (torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack() or
+                torch._C._get_tracing_state() is not None or
+                torch._C._functorch.peek_interpreter_stack() is not None or
+                torch.autograd.forward_ad._current_level >= 0 or torch._C._autograd._profiler_enabled()):
+            return False
+        dev = torch._C._cuda_getDevice() if torch.cuda.is_initialized() else -1
+    except AttributeError:
         return False
     for i in ints:
         if not -(1 << 63) <= i < 1 << 63:
             return False
-    dev = torch._C._cuda_getDevice() if torch.cuda.is_initialized() else -1
     for x, dtype in zip(xs, dtypes):
         if (type(x) is not torch.Tensor or x.dtype not in dtype or not x.is_cuda or x.get_device() != dev or
                 x.requires_grad or not x.is_contiguous() or x.is_neg()):
