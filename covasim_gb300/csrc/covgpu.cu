@@ -1163,12 +1163,18 @@ constexpr int DYN_WARPS = 8;  // warps per thread block
 // dependent loads, so more warps only pay where the chip would idle (ms a 100-day run
 // with one / two / four / eight: 20,000 agents 3.19, 3.00, 2.86, 2.79; 100,000 3.30,
 // 3.11, 3.09, 3.25; 200,000 4.15, 3.99, 3.99, -; 300,000 with testing, 120 days, 6.82,
-// 6.56, -, -; 1M, 180 days, 14.9, 15.5, 17.7, 20.0).
+// 6.56, -, -; 1M, 180 days, 14.9, 15.5, 17.7, 20.0). The walk of all stored layers in a
+// launch of its own has no redrawn layer's warps beside it, and a warp's edges are its
+// work on busy days: WALK_SPLIT_TARGET, about forty an SM (a 100-day run with tracing,
+// a tenth of the symptomatic tested daily / a hundredth, with 1520 / 6080 warps, and
+// streamed: random 530,000 agents 6.60, 8.97 / 6.35, 7.71, streamed 7.05, 7.62; 700,000
+// 7.64, 10.13 / 7.52, 9.34, streamed 8.45, 9.22; hybrid 1M 10.55, 15.32 / 10.36, 14.96,
+// streamed 13.95, 16.28).
 constexpr int AB_WORDS = AGENT_THREADS / 32;  // source-bitmap words of an agent block
-constexpr int64_t SPLIT_TARGET = 1520;
-inline int source_split(const covgpu_state* st) {
+constexpr int64_t SPLIT_TARGET = 1520, WALK_SPLIT_TARGET = 6080;
+inline int source_split(const covgpu_state* st, int64_t target) {
   int split = 1;
-  while (split < AB_WORDS && st->n_agent_blocks * split < SPLIT_TARGET) split *= 2;
+  while (split < AB_WORDS && st->n_agent_blocks * split < target) split *= 2;
   return split;
 }
 
@@ -1613,10 +1619,13 @@ __global__ void __launch_bounds__(DYN_WARPS * 32, COVGPU_DYN_MIN_BLOCKS) k_sourc
   pdl_trigger();
 }
 
+// every stored layer is walked on every day: the tile pass has nothing to do
+inline bool walk_all(const covgpu_state* st) { return st->src_walk == COVGPU_WALK_ALL; }
+
 // dependent: launched as a dependent of the stream's previous kernel
 template <bool LIK>
 void launch_source_lik(const covgpu_state* st, int t, cudaStream_t s, bool dyn, bool walk, bool dependent) {
-  const int split = source_split(st);
+  const int split = source_split(st, !LIK && !dyn && walk_all(st) ? WALK_SPLIT_TARGET : SPLIT_TARGET);
   const unsigned g = (unsigned)((split * st->n_agent_blocks + DYN_WARPS - 1) / DYN_WARPS);
   const unsigned grid = dyn && walk ? 2 * g : g;
   void (*k)(covgpu_state, int, int) = dyn && walk ? k_source_pass<LIK, true, true>
@@ -1761,9 +1770,6 @@ int launch_stored_pass(const covgpu_state* st, int t, cudaStream_t s, bool with_
   const int rc = launch_status();
   return (rc || !with_walk) ? rc : launch_source_pass(st, t, s, false, true, false);
 }
-
-// every stored layer is walked on every day: the tile pass has nothing to do
-inline bool walk_all(const covgpu_state* st) { return st->src_walk == COVGPU_WALK_ALL; }
 
 // the stored layers' tiles, then the redrawn layers' sources (parts: 0 both, 1 or 2
 // one of them); the walk of the stored layers goes with the redrawn layers' pass

@@ -262,42 +262,63 @@ def ili_agents(seed, t, n, n_ili):
 
 
 # When the stored layers are walked from the day's sources (covgpu_state.src_walk;
-# results are the same either way). BatchState.src_walk is the threshold k of a
-# state with a redrawn layer (SRC_WALK), or without one of a state whose stored
-# edges make a day's stream long (SRC_WALK_BIG, from SRC_WALK_MIN_EDGES edges in one
-# sim, SRC_WALK_MIN_EDGES_BATCH in several); both build the agent index the walk
-# needs, as tracing does. Until set_src_walk asks for a threshold, _walk_mode refines
-# it from sizes once every stored layer has its index (ms a run; "every day" also
-# leaves out the tile pass's launch):
-# * one sim without a redrawn layer: below 1/16 (100-120 days, streamed / every day /
-#   1/16: random 700,000 agents, 7M edges, 8.38, -, 8.13; 1M 11.7, -, 10.8; 2M 23.0,
-#   20.9, 17.8; hybrid 1M, 17.8M edges, 15.9, 15.7, 14.0; building the index takes
-#   0.5 ms at 1M); with tracing, which has the index anyway, every day from
-#   SRC_WALK_TRACE_AGENTS (hybrid 20,000 agents 3.45, 3.72, 4.08; 100,000 3.81, 3.79,
-#   4.19; 300,000 5.23, 5.06, 5.46; 1M 10.97, 9.24, 9.69; 4M 18.0, 10.2, 10.3);
-# * several: every day (24 to 96 random sims, streamed / every day / 1/64: 17M edges
-#   16.0, 18.1, 16.9; 30M 24.6, 24.6, 24.6; 43M 33.1, 29.2, 31.7; 115M -, 83.5, 106);
-# * a redrawn layer and testing: one sim walks every day, one launch with the redrawn
-#   layer's pass instead of a fork and join of two (100-120 days, every day / 1/16 /
-#   1/128: 200,000 agents 6.40, 6.76, 6.57; 300,000 6.85, 7.25, 7.15; 800,000 8.83, 9.10,
-#   8.79; 1.5M 12.97, 13.30, 13.72; 6M, 60 days, 15.8, 15.9, 16.5; 10M, three variants,
-#   105.2, 105.4, 111.3); several do below SRC_WALK_ALL_AGENTS agents, else SRC_WALK
-#   (16 of 20,000 7.12, 7.45, 7.30; 8 of 60,000 7.91, 8.25, 7.87; 48 of 20,000 12.9,
-#   13.3, 12.6);
-# * a redrawn layer without testing: below 1/32, the stream beside the redrawn layer's
-#   pass being faster on the busy days (every day / 1/16 / 1/32 / 1/128: 30,000 agents
-#   3.51, 3.43, 3.41, 3.38; 300,000 5.75, 5.59, 5.55, 5.55; 1M, 150 days, 14.75, 13.25,
-#   13.12, 13.27; 3M, 100 days, 23.8, 21.4, 21.5, 22.0);
-# * with the likelihood, whose walk takes the layers one after another, SRC_WALK
-#   (100,000 agents: 7.96 ms, 8.44 every day).
+# results are the same either way). BatchState.src_walk says whether the agent index
+# that the walk needs is built (tracing builds it too): SRC_WALK for a state with a
+# redrawn layer, SRC_WALK_BIG for one without whose stored edges make a day's stream
+# long (SRC_WALK_MIN_EDGES edges in one sim, SRC_WALK_MIN_EDGES_BATCH in several). They
+# are also the threshold with the likelihood, whose walk takes the layers one after
+# another (100,000 agents: 7.96 ms, 8.44 every day), and of large batches with testing
+# and a redrawn layer. Else, until set_src_walk asks for one, _walk_mode chooses from
+# sizes once every stored layer has its index. What testing does to the epidemic decides
+# the walk's work, and sizes cannot tell: measured with 10% of the symptomatic tested a
+# day and their contacts traced from day 0 (A), the same from mid-run (B), 1% tested (C)
+# and 10% until day 30, untraced (D); peaks of 5, 6, 19 and 26% infectious (ms a run of
+# 80 to 120 days; "every day" also leaves out the tile pass's launch):
+# * a redrawn layer and testing, fewer than SRC_WALK_ALL_AGENTS agents in all: every day,
+#   one launch with the redrawn layer's pass instead of a fork and join of two, faster
+#   where testing keeps the epidemic small and up to 7% slower where it does not (every
+#   day / 1/32 / 1/128: 20,000 agents A 3.24, 3.27, 3.23, D 2.71, 2.68, 2.67; 150,000 A
+#   5.69, 5.94, 5.95, D 5.21, 5.25, 5.24; 300,000 A 6.78, 7.05, 7.06, B 6.59, 6.76, 6.76,
+#   C 7.53, 7.34, 7.38, D 6.53, 6.26, 6.27; 16 sims of 20,000 A 5.55, 5.82, 5.78, D 5.21,
+#   5.00, 5.00); with more agents several sims below SRC_WALK (48 of 20,000 C 12.13,
+#   10.73, 10.61; 3 of 200,000 C 6.40, 5.95, 5.99);
+# * a redrawn layer, else: below 1/32, one sim from SRC_WALK_LARGE agents 1/16, the
+#   stream beside the redrawn layer's pass being much faster on busy days (every day /
+#   1/16 / 1/32 / 1/128, with testing: 420,000 agents A 8.35, -, 8.39, 8.36, C 10.17, -,
+#   8.99, 8.99, D 8.99, -, 7.67, 7.63; 1M A 10.48, -, 10.62, 10.70, C 13.38, -, 12.17,
+#   12.19, D 11.91, -, 10.51, 10.55; 4M A 27.42, 27.78, 28.20, 29.21, C 37.25, 34.59,
+#   34.66, 35.36; 12M A 70.72, 71.27, 73.18, 76.47, C 101.07, 95.87, 96.33, 98.38; without:
+#   20,000 2.95, 2.91, 2.88, 2.86; 1M 10.72, 9.24, 9.18, 9.23; 8M 37.34, 35.53, 35.82,
+#   37.17; 48 sims of 20,000 12.27, 10.39, 10.12, 10.04);
+# * stored layers only, one sim with testing: with at most SRC_WALK_FEW_EDGES edges an
+#   agent every day from SRC_WALK_FEW_AGENTS agents, with more from SRC_WALK_MANY_AGENTS
+#   and below 1/32 from SRC_WALK_TRACE_AGENTS; else streamed (every day / 1/32 / streamed:
+#   random, 10 edges, 150,000 agents A 3.74, 4.19, 3.85, C 4.40, 4.67, 4.29; 300,000 A
+#   5.08, 5.42, 5.32, C 5.59, 5.65, 5.51; 530,000 A 6.35, 6.77, 7.05, C 7.71, 7.55, 7.62; 1M
+#   A 9.15, 9.79, 11.24, C 11.79, 11.68, 12.66; hybrid, 17.75 edges, 300,000 C 6.82, 6.67,
+#   6.54; 400,000 A 6.65, 7.37, 7.50, C 8.72, 8.00, 8.09; 700,000 A 8.79, 9.35, 10.32, C
+#   11.69, 10.76, 11.40; 900,000 A 8.91, 9.67, 11.85, C 13.14, 12.61, 13.97; 4M A 27.96,
+#   30.85, 50.30, C 44.73, 42.75, 56.40);
+# * stored layers only, one sim without testing: below 1/16 (100-120 days, streamed /
+#   every day / 1/16: random 700,000 agents, 7M edges, 8.38, -, 8.13; 1M 11.7, -, 10.8;
+#   2M 23.0, 20.9, 17.8; hybrid 1M, 17.8M edges, 15.9, 15.7, 14.0; building the index
+#   takes 0.5 ms at 1M);
+# * stored layers only, several sims: every day (24 to 96 random sims, streamed / every
+#   day / 1/64: 17M edges 16.0, 18.1, 16.9; 30M 24.6, 24.6, 24.6; 43M 33.1, 29.2, 31.7;
+#   115M -, 83.5, 106; with testing, 30 of 100,000 hybrid agents, A 25.51, 16.89, 21.4,
+#   C 29.59, 24.47, 26.2; 12 of 300,000 C 32.59, 23.39, 27.0).
 SRC_WALK = 128
 SRC_WALK_REDRAWN = 32
-SRC_WALK_ALL_AGENTS = 400_000
+SRC_WALK_LARGE = 4_000_000
+SRC_WALK_ALL_AGENTS = 350_000
 SRC_WALK_BIG = 64
 SRC_WALK_MIN_EDGES = 10_000_000
 SRC_WALK_MIN_EDGES_BATCH = 30_000_000
 SRC_WALK_ONE = 16
-SRC_WALK_TRACE_AGENTS = 150_000
+SRC_WALK_FEW_EDGES = 12
+SRC_WALK_FEW_AGENTS = 150_000
+SRC_WALK_MANY_AGENTS = 900_000
+SRC_WALK_TRACE_AGENTS = 400_000
 
 
 def parse_edge_tile(choice):
@@ -787,14 +808,20 @@ class BatchState:
         indexed = all(rec.dynamic or rec.rp1 for rec in self.segments)
         if self._walk_default and indexed and not self.lik_active:
             dynamic = any(rec.dynamic for rec in self.segments)
-            if dynamic and self.has_testing:
-                k = -1 if len(self.specs) == 1 or self.n < SRC_WALK_ALL_AGENTS else SRC_WALK
+            if dynamic and self.has_testing and self.n < SRC_WALK_ALL_AGENTS:
+                k = -1
+            elif dynamic and len(self.specs) > 1:
+                k = SRC_WALK if self.has_testing else SRC_WALK_REDRAWN
             elif dynamic:
-                k = SRC_WALK_REDRAWN
+                k = SRC_WALK_ONE if self.n >= SRC_WALK_LARGE else SRC_WALK_REDRAWN
             elif len(self.specs) > 1:
                 k = -1 if k else 0
             elif self.has_testing:
-                k = -1 if self.n >= SRC_WALK_TRACE_AGENTS else 0
+                few = sum(rec.n_edges for rec in self.segments) <= SRC_WALK_FEW_EDGES * self.n
+                if self.n >= (SRC_WALK_FEW_AGENTS if few else SRC_WALK_MANY_AGENTS):
+                    k = -1
+                else:
+                    k = SRC_WALK_REDRAWN if self.n >= SRC_WALK_TRACE_AGENTS else 0
             else:
                 k = SRC_WALK_ONE
         return L.WALK_ALL if indexed and k == -1 else k
