@@ -51,13 +51,13 @@ RECORDED_CUM_INFECTIONS = {(1_000_000, 180, 1): 1_055_079}
 
 MEASURED_NCU = {
     ('agent_step', 1_000_000): {
-        'dram_bytes': 75_929_088, 'issue_active': 0.625, 'bound': 'issue',
-        'note': 'ncu section capture, day 85 of the 1M-agent run: 75.9 MB of DRAM traffic against 88 MB '
+        'dram_bytes': 75_626_752, 'issue_active': 0.624, 'bound': 'issue',
+        'note': 'ncu section capture, day 85 of the 1M-agent run: 75.6 MB of DRAM traffic against 88 MB '
                 'algorithmic; instruction issue 62% busy, 38.9 M warp instructions for 1M agents (with the '
                 'severe efficacy, stored on a sequence\'s last day only), so the pass '
                 'is issue-bound on the float-float efficacies, not HBM-bound'},
     ('edge_stored', 1_000_000): {
-        'dram_bytes': 83_339_008, 'issue_active': 0.574, 'bound': 'latency',
+        'dram_bytes': 82_925_760, 'issue_active': 0.600, 'bound': 'latency',
         'note': 'ncu section capture, day 85 (one-wave pass, 2048-edge tiles): 83 MB of DRAM traffic (the 62 MB '
                 'of stored edge lists and the candidates\' records); long-scoreboard stalls dominate'},
 }

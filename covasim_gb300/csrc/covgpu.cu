@@ -1405,10 +1405,10 @@ __device__ __forceinline__ void dyn_body(const covgpu_state& st, int t, int64_t 
 // source is p2, as in the tile pass), and the queue drains through edge_try 32
 // candidates at a time, whatever their layers (the likelihood's sums are kept per
 // layer, so its walk takes one layer after another). It waits on memory: at the
-// peak of a 1M-agent hybrid epidemic (about a quarter infectious) 98 us, against
-// 57 us for the tile pass, whose reads are streams; below a tenth infectious it is
-// the cheaper one, and in a launch with the redrawn layers' draws at every size
-// up to some hundred thousand agents.
+// peak of a 1M-agent hybrid epidemic (about a quarter infectious) 95 us, against
+// 57 us for the tile pass, whose reads are streams; below about 1/32 infectious it is
+// the cheaper one. Which sizes are walked on every day stands beside SRC_WALK in
+// state.py.
 constexpr int SRC_WARPS = 8;
 constexpr int WALK_U = 2;  // 1 and 4 within 1% (4 slower)
 constexpr int WQ_CAP = 32 + 32 * WALK_U;  // fewer than 32 left over + one round's pushes

@@ -740,9 +740,9 @@ class BatchState:
         self._tile_segments()
 
     def _trace_index(self, rec, sp, off, n_edges):
-        """Agent index of a stored layer (covgpu_trace_index), built now when the sim
-        traces (tracing visits the traced agents' edges through it), else when the
-        walk from the sources is switched on (set_src_walk)."""
+        """Agent index of a stored layer (covgpu_agent_index), built now when the sim
+        traces (tracing visits the traced agents' edges through it) or the state's
+        default is to walk from the sources, else when set_src_walk asks for the walk."""
         if n_edges < 1 or n_edges > 0xFFFFFFFF:
             return []
         T = sp.testing
